@@ -33,7 +33,7 @@ REFERENCE_SRC = "/root/reference"
 def build_reference() -> bool:
     """Build SFbox from the reference's own sources into oracle/_ref (sfbox and
     the sfref driver) when the sources are present; False otherwise."""
-    if not os.path.isdir(REFERENCE_SRC):
+    if not os.path.exists(os.path.join(REFERENCE_SRC, "SF_Box.cpp")):
         return False
     subprocess.check_call(["make", "-s", "-j8", "-C", REFBUILD, f"REF={REFERENCE_SRC}"])
     return True
