@@ -8,7 +8,7 @@
 #include <cstring>
 #include <vector>
 #include "sfgpu_batch_kernel.cuh"
-#include "sfgpu_system.h"
+#include "sfgpu_group.h"
 
 using namespace sfb;
 
@@ -23,6 +23,9 @@ struct sfgpu_batch {
     int m = 10, block = 256;
     size_t stage_bytes = 0;         // dynamic shared memory per block (staged G)
     bool wide = false;              // some instance needs batch_diis_kernel_t<true>
+    bool grouped = false;           // every instance runs in the cluster engine, with this shape
+    GroupShape shape;
+    int clusters = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -88,6 +91,53 @@ static int configure_stage(sfgpu_batch *b, bool allow) {
     return SFGPU_OK;
 }
 
+// The cluster engine takes a batch whose instances it all accepts on lattices
+// of one kind.  2D blocks per instance: with enough instances to fill the
+// chip, about 2048 sites a block (fewer blocks idle less in halo exchanges,
+// more let two blocks share an SM and hide them); 296 cylinders of 128 x 128
+// to 1e-11: 172 ms with 8 blocks of 256 threads, 176 with 4 of 512, 218 with 16
+// of 256, and 231 in the one-block-per-instance kernel.  With fewer instances
+// the SMs left over go to their clusters.
+static void configure_group(sfgpu_batch *b) {
+    const sfgpu_system *s0 = b->sys[0];
+    const int n = (int)b->sys.size();
+    long sites = 1;
+    for (auto *s : b->sys) {
+        const DLat &L = s->H.L;
+        if (!s->group || L.grad != s0->H.L.grad || (L.cyl != 0) != (s0->H.L.cyl != 0)) return;
+        if (L.grad == 2) sites = std::max(sites, (long)(L.Md[0] - 2) * (L.Md[1] - 2));
+    }
+    int C = 1, threads = 256;
+    if (s0->H.L.grad == 2) {
+        while (C < 8 && sites > 2048L * C) C *= 2;
+        const int base = C;
+        while (C < 16 && 2L * C * n <= 148) C *= 2;
+        if (C > base) threads = 512;
+    } else if (n <= 148) {
+        C = 2;   // 1D: one block an SM, whose shared memory the chain's slices may fill
+    }
+    GroupShape big;
+    for (auto *s : b->sys) {
+        GroupShape g;
+        if (!group_shape(s, C, threads, b->m, &g)) return;
+        big.J = std::max(big.J, g.J);
+    }
+    for (auto *s : b->sys) {
+        GroupShape g;
+        group_shape(s, C, threads, b->m, &g);
+        big.dim = g.dim;
+        big.curved = g.curved;
+        big.C = std::max(big.C, g.C);
+        big.threads = std::max(big.threads, g.threads);
+        big.smem = std::max(big.smem, g.smem);
+    }
+    const int most = group_max_clusters(big, true);
+    if (most < 1) return;
+    b->shape = big;
+    b->clusters = std::min(n, most);
+    b->grouped = true;
+}
+
 extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, sfgpu_batch **out) {
     if (!out || !descs || n < 1) return SFGPU_ERR_INVALID;
     *out = nullptr;
@@ -118,6 +168,7 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
         sfgpu_system *s = new sfgpu_system();
         s->stream = b->stream;
         rc = s->setup(&descs[i]);
+        if (!rc) rc = s->setup_group();
         if (!rc && (s->nseg > kResMax || s->nclass > kResMax)) rc = SFGPU_ERR_UNSUPPORTED;   // site_residual registers
         if (rc) { delete s; break; }
         b->sys.push_back(s);
@@ -132,33 +183,8 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
     for (int i = 0; i < n && !rc; i++) {
         sfgpu_system *s = b->sys[i];
         InstDesc &I = b->desc_h[i];
-        memset(&I, 0, sizeof(I));
-        I.L = s->H.L;
-        I.M = s->M; I.nseg = s->nseg; I.nmol = s->nmol; I.nclass = s->nclass; I.nsites = s->nsites;
-        I.solvent = s->solvent; I.nvar = (long long)s->nvar;
-        for (int q = 0; q < s->nseg; q++) {
-            I.freedom[q] = s->freedom[q];
-            I.class_of[q] = s->class_of[q];
-            I.range[q] = s->d_range[q];
-            I.gfull[q] = s->d_gfull[q]; I.gseg[q] = s->d_gseg[q]; I.phi[q] = s->d_phi[q];
-        }
-        for (int c = 0; c < s->nclass; c++) I.rep[c] = s->rep_of_class[c];
-        I.ct = s->ct;
-        memcpy(I.frac, s->bp.frac, sizeof(I.frac));
-        I.jmap = s->d_jmap; I.sites = s->d_sites; I.w_gn = s->d_wgn;
-        for (int q = 0; q < s->nmol; q++) {
-            const HMol &o = s->mols[q];
-            IMol &im = I.mol[q];
-            im.N = o.N; im.type = o.type; im.sym = o.sym; im.freedom = o.freedom; im.pinned = o.pinned;
-            im.solvent = (q == s->solvent); im.phibulk = o.phibulk; im.theta = o.theta;
-            im.nused = (int)o.used.size();
-            for (int a = 0; a < im.nused; a++) im.used[a] = o.used[a];
-            for (int a = 0; a < s->nseg; a++) im.phi[a] = o.d_phi[a];
-            int *dseg = nullptr;
-            if ((rc = balloc(b, (void **)&dseg, sizeof(int) * o.N))) break;
-            if (cudaMemcpy(dseg, o.seg.data(), sizeof(int) * o.N, cudaMemcpyHostToDevice) != cudaSuccess) { rc = SFGPU_ERR_CUDA; break; }
-            im.seg = dseg;
-        }
+        fill_inst_desc(s, &I);
+        rc = s->upload_chains(&I);
         if (rc) break;
         {   // force ensembles: step weights per molecule
             std::vector<sfk::ForceW> fw(2 * s->nmol);
@@ -179,7 +205,6 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
             }
             I.fw = dfw;
         }
-        I.gi = s->d_gi; I.ginv0 = s->d_ginv[0]; I.ginv1 = s->d_ginv[1];
         const size_t iv = s->nvar;
         I.x = b->d_xall + b->offset[i];
         if ((rc = balloc(b, (void **)&I.x0, sizeof(double) * iv)) || (rc = balloc(b, (void **)&I.g, sizeof(double) * iv)) ||
@@ -197,6 +222,7 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
     // on the uneven 1D sweep, where 384 beat 256 by 4.5 % and 32..128 lost)
     b->block = maxM >= 4096 ? 1024 : (maxM >= 1024 ? 512 : (maxM >= 384 ? 384 : 256));
     if ((rc = configure_stage(b, true))) { delete b; return rc; }
+    configure_group(b);
     *out = b;
     return SFGPU_OK;
 }
@@ -229,7 +255,7 @@ extern "C" int sfgpu_batch_set_stream(sfgpu_batch *b, void *stream) {
 // Launch shape of the persistent kernel: threads per block (32..1024, a
 // multiple of 32) and whether instances stage G (and the 1D slices) in
 // shared memory.  By default 1024/512/256 threads by lattice size and
-// staging on.
+// staging on.  Batches of the cluster engine keep the engine's own shape.
 extern "C" int sfgpu_batch_set_launch(sfgpu_batch *b, int threads, int stage) {
     if (!b || threads < 32 || threads > 1024 || threads % 32) return SFGPU_ERR_INVALID;
     SFGPU_CUDA_TRY(cudaStreamSynchronize(b->stream));
@@ -264,6 +290,13 @@ extern "C" int sfgpu_batch_solve_resident(sfgpu_batch *b, double tol, int maxit,
         SFGPU_CUDA_TRY(cudaEventCreate(&b->ev1));
     }
     SFGPU_CUDA_TRY(cudaEventRecord(b->ev0, st));
+    if (b->grouped) {
+        const int rc = group_diis(b->shape, b->d_desc, n, b->clusters, b->d_queue, b->m, eta, tol, maxit, b->d_status,
+                                  b->d_iters, b->d_err, st);
+        if (rc) return rc;
+        SFGPU_CUDA_TRY(cudaEventRecord(b->ev1, st));
+        return SFGPU_OK;
+    }
     batch_kernel(b)<<<grid, b->block, b->stage_bytes, st>>>(b->d_desc, n, b->d_queue, b->m, eta, tol, maxit,
                                                   b->d_status, b->d_iters, b->d_err);
     SFGPU_CUDA_TRY(cudaGetLastError());

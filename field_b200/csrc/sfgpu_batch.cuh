@@ -20,6 +20,7 @@ struct IMol {
     int N, type, sym, freedom, pinned, solvent, nused;
     int used[SFGPU_MAX_SEG];
     const int *seg;                 // device: segment of each chain position
+    const int *runf, *runb;         // first position after / last before the run of equal segments it lies in
     double *phi[SFGPU_MAX_SEG];     // per segment, nullptr when unused
     double phibulk, theta;
 };
@@ -48,6 +49,14 @@ struct InstDesc {
     // forward and backward step weights are fw[2m], fw[2m + 1]
     int fmask;
     const sfk::ForceW *fw;
+    // the cluster engine (sfgpu_group.cuh): per site r the site it copies
+    // (lat_map) and that site's iteration index (jmap), ceil(M / 256) partial
+    // sums per molecule, and where the last evaluation's scalars go (or null)
+    const int *smap, *jall;
+    int need;                       // bit i: some class interacts with segment i
+    double *wpart, *slices1;        // slices1: 1D stored slices in whole warps
+    sfk::MolScal *scal_out;
+    double *phib_out, *chib_out;
 };
 
 struct BlockShared {
@@ -380,13 +389,13 @@ __device__ inline void molecule_phi_block(const InstDesc &I, int m, BlockShared 
 }
 
 // f at iteration site j (lattice site z) of SF_Solve::GetResiduals
-// (SF_Solve.cpp:527-591) once phi and the bulk terms (sh.chib) are known.
+// (SF_Solve.cpp:527-591) once phi and the bulk terms (chib) are known.
 // Segment types and classes are bounded by kResMax so that the per-site
 // contact averages and potentials stay in registers; the sums run in the
 // same order as the single-system kernel.
 constexpr int kResMax = 8;
 template <bool kWide>
-__device__ __forceinline__ void site_residual(const InstDesc &I, const BlockShared &sh, int j, double *f) {
+__device__ __forceinline__ void site_residual(const InstDesc &I, const double *chib, int j, double *f) {
     const DLat &L = I.L;
     const int z = I.sites[j];
     const int nseg = I.nseg, ncl = I.nclass;
@@ -420,7 +429,7 @@ __device__ __forceinline__ void site_residual(const InstDesc &I, const BlockShar
             if (xx != 0) ci += xx * rho[i];
         }
         v -= ci / phit;
-        v += sh.chib[c];
+        v += chib[c];
         u[c] = v;
         av += v;
     }
@@ -486,7 +495,7 @@ __device__ inline void residual_block(const InstDesc &I, const double *x, double
         }
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < I.nsites; j += blockDim.x) site_residual<kWide>(I, sh, j, f);
+    for (int j = threadIdx.x; j < I.nsites; j += blockDim.x) site_residual<kWide>(I, sh.chib, j, f);
     __syncthreads();
 }
 

@@ -8,7 +8,7 @@
 #include <cstring>
 #include <vector>
 #include <algorithm>
-#include "sfgpu_system.h"
+#include "sfgpu_group.h"
 
 using namespace sfk;
 
@@ -71,6 +71,7 @@ extern "C" int sfgpu_solve_diis(sfgpu_system *s, double *x_host, double tol, int
                                 double eta, int *iterations, double *final_error) {
     if (!s || !x_host) return SFGPU_ERR_INVALID;
     if (m < 1 || m > 64 || !(eta > 0) || maxit < 0) return SFGPU_ERR_INVALID;
+    if (s->group_shape_ && m <= sfb::kMaxHist) return s->solve_group(x_host, tol, maxit, m, eta, iterations, final_error);
     const size_t iv = s->nvar;
     cudaStream_t st = s->stream;
     DiisWork w;

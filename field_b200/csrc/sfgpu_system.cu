@@ -10,7 +10,7 @@
 #include <vector>
 #include <algorithm>
 #include "sfgpu_kernels.cuh"
-#include "sfgpu_system.h"
+#include "sfgpu_group.h"
 
 static thread_local char g_errmsg[512] = "";
 
@@ -319,6 +319,8 @@ static bool chi_cols_equal(const std::vector<double> &chi, int ns, int a, int b)
 }
 
 sfgpu_system::~sfgpu_system() {
+    delete group_shape_;
+    if (d_diis) cudaFree(d_diis);
     if (a_store) cudaFree(a_store);
     if (a_ring) cudaFree(a_ring);
     if (a_tree) cudaFree(a_tree);
@@ -555,6 +557,7 @@ int sfgpu_system::setup(const sfgpu_system_desc *d) {
     nsites = (int)sites_h.size();
     nvar = (size_t)nsites * nclass;
     if (nsites == 0) return fail(SFGPU_ERR_INVALID, "no sites carry iteration variables");
+    jmap_h = jmap;
     if ((rc = setup_charges(d, jmap))) return rc;
 
     // device buffers
@@ -643,6 +646,169 @@ int sfgpu_system::setup(const sfgpu_system_desc *d) {
         for (int m = 0; m < nmol; m++) bp.frac[i * SFGPU_MAX_SEG + m] = (double)mols[m].count[i] / mols[m].N;
     if (d->overflow_protection) return setup_logspace();
     return SFGPU_OK;
+}
+
+void fill_inst_desc(const sfgpu_system *s, sfb::InstDesc *out) {
+    sfb::InstDesc &I = *out;
+    memset(&I, 0, sizeof(I));
+    I.L = s->H.L;
+    I.M = s->M; I.nseg = s->nseg; I.nmol = s->nmol; I.nclass = s->nclass; I.nsites = s->nsites;
+    I.solvent = s->solvent; I.nvar = (long long)s->nvar;
+    for (int q = 0; q < s->nseg; q++) {
+        I.freedom[q] = s->freedom[q];
+        I.class_of[q] = s->class_of[q];
+        I.range[q] = s->d_range[q];
+        I.gfull[q] = s->d_gfull[q]; I.gseg[q] = s->d_gseg[q]; I.phi[q] = s->d_phi[q];
+    }
+    for (int c = 0; c < s->nclass; c++) I.rep[c] = s->rep_of_class[c];
+    I.ct = s->ct;
+    memcpy(I.frac, s->bp.frac, sizeof(I.frac));
+    I.jmap = s->d_jmap; I.sites = s->d_sites; I.w_gn = s->d_wgn;
+    for (int q = 0; q < s->nmol; q++) {
+        const HMol &o = s->mols[q];
+        sfb::IMol &im = I.mol[q];
+        im.N = o.N; im.type = o.type; im.sym = o.sym; im.freedom = o.freedom; im.pinned = o.pinned;
+        im.solvent = (q == s->solvent); im.phibulk = o.phibulk; im.theta = o.theta;
+        im.nused = (int)o.used.size();
+        for (int a = 0; a < im.nused; a++) im.used[a] = o.used[a];
+        for (int a = 0; a < s->nseg; a++) im.phi[a] = o.d_phi[a];
+    }
+    I.slices1 = s->d_slices1;
+    I.gi = s->d_gi; I.ginv0 = s->d_ginv[0]; I.ginv1 = s->d_ginv[1];
+    for (int i = 0; i < s->nseg; i++)
+        for (int c = 0; c < s->nclass; c++)
+            if (s->ct.chi[s->rep_of_class[c] * SFGPU_MAX_SEG + i] != 0) I.need |= 1 << i;
+    I.smap = s->d_smap; I.jall = s->d_jall; I.wpart = s->d_wpart;
+}
+
+// every molecule's segments and their runs on the device
+int sfgpu_system::upload_chains(sfb::InstDesc *I) {
+    std::vector<int> all;
+    std::vector<size_t> at(nmol);
+    for (int q = 0; q < nmol; q++) {
+        const std::vector<int> &s = mols[q].seg;
+        const int n = (int)s.size();
+        std::vector<int> f(n), b(n);
+        for (int t = n - 1; t >= 0; t--) f[t] = (t + 1 < n && s[t + 1] == s[t]) ? f[t + 1] : t + 1;
+        for (int t = 0; t < n; t++) b[t] = (t > 0 && s[t - 1] == s[t]) ? b[t - 1] : t - 1;
+        at[q] = all.size();
+        all.insert(all.end(), s.begin(), s.end());
+        all.insert(all.end(), f.begin(), f.end());
+        all.insert(all.end(), b.begin(), b.end());
+    }
+    int *d = nullptr;
+    const int rc = alloc_i(&d, all.size());
+    if (rc) return rc;
+    SFGPU_CUDA_TRY(cudaMemcpy(d, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice));
+    for (int q = 0; q < nmol; q++) {
+        const size_t n = mols[q].seg.size();
+        I->mol[q].seg = d + at[q];
+        I->mol[q].runf = d + at[q] + n;
+        I->mol[q].runb = d + at[q] + 2 * n;
+    }
+    return SFGPU_OK;
+}
+
+// Where the cluster engine takes the system: its index maps, its descriptor
+// on the device and its launch shape for one system alone.
+int sfgpu_system::setup_group() {
+    if (!group_eligible(this)) return SFGPU_OK;
+    int rc;
+    std::vector<int> smap(M), jall(M);
+    for (int z = 0; z < M; z++) { smap[z] = lat_map(H.L, z); jall[z] = jmap_h[smap[z]]; }
+    if ((rc = alloc_i(&d_smap, M)) || (rc = alloc_i(&d_jall, M)) ||
+        (rc = alloc_d(&d_wpart, (size_t)nmol * ((M + 255) / 256))))
+        return rc;
+    SFGPU_CUDA_TRY(cudaMemcpy(d_smap, smap.data(), sizeof(int) * M, cudaMemcpyHostToDevice));
+    SFGPU_CUDA_TRY(cudaMemcpy(d_jall, jall.data(), sizeof(int) * M, cudaMemcpyHostToDevice));
+    if (H.L.grad == 1) {
+        // stored slices of whole warps, for chains that shared memory does not
+        // take; apart from d_gi, whose slices' boundary entries stay 0 for the
+        // derivatives' sweeps
+        size_t n = 0;
+        for (const auto &o : mols)
+            if (o.type != 0) n = std::max(n, (size_t)(o.sym ? o.N / 2 : o.N) * sfg::slice1d(H.L.Md[0] - 2));
+        if ((rc = alloc_d(&d_slices1, n))) return rc;
+    }
+    // surface layers hold 0 in every profile: the contact averages read them
+    // where the boundary copies are written in the same phase
+    for (int i = 0; i < nseg; i++) {
+        if (freedom[i] == SFGPU_SEG_FROZEN) continue;
+        SFGPU_CUDA_TRY(cudaMemset(d_phi[i], 0, sizeof(double) * M));
+        for (const auto &o : mols)
+            if (o.d_phi[i]) SFGPU_CUDA_TRY(cudaMemset(o.d_phi[i], 0, sizeof(double) * M));
+    }
+    group = true;
+    return SFGPU_OK;
+}
+
+// the launch shape of one system alone, and its descriptor on the device
+int sfgpu_system::setup_group_single() {
+    GroupShape sh;
+    bool ok = false;
+    // one system alone leaves the chip idle: as many blocks as a cluster has,
+    // of 256 sites at least (64 x 64: 8 and 16 blocks take the same time)
+    const long sites = (long)(H.L.Md[0] - 2) * (H.L.grad == 2 ? H.L.Md[1] - 2 : 1);
+    for (int blocks = (int)std::max(2L, std::min(16L, (sites + 255) / 256)); !ok && blocks >= 2; blocks = (blocks + 1) / 2) {
+        ok = group_shape(this, blocks, 512, 0, &sh) && group_max_clusters(sh, false) > 0 &&
+             group_max_clusters(sh, true) > 0;
+        if (blocks == 2) break;
+    }
+    if (!ok) return SFGPU_OK;
+    sfb::InstDesc I;
+    fill_inst_desc(this, &I);
+    int rc;
+    double *p = nullptr, *p2 = nullptr;
+    const size_t nd = (sizeof(sfb::InstDesc) + 7) / 8;
+    if ((rc = upload_chains(&I)) || (rc = alloc_d(&p, nd)) || (rc = alloc_d(&p2, nd)) ||
+        (rc = alloc_i(&d_diis_int, 4)))
+        return rc;
+    I.scal_out = (MolScal *)d_scal;
+    I.phib_out = d_phib;
+    I.chib_out = d_chib;
+    d_inst = (sfb::InstDesc *)p;
+    d_inst_solve = (sfb::InstDesc *)p2;
+    SFGPU_CUDA_TRY(cudaMemcpy(d_inst, &I, sizeof(I), cudaMemcpyHostToDevice));
+    group_shape_ = new GroupShape(sh);
+    return SFGPU_OK;
+}
+
+// Pure_DIIS of one system in one launch (group_diis_kernel)
+int sfgpu_system::solve_group(double *x, double tol, int maxit, int m, double eta, int *iterations,
+                              double *final_error) {
+    cudaStream_t st = stream;
+    if (diis_m < m) {
+        if (d_diis) { SFGPU_CUDA_TRY(cudaStreamSynchronize(st)); SFGPU_CUDA_TRY(cudaFree(d_diis)); }
+        d_diis = nullptr;
+        diis_m = 0;
+        const int rc = dalloc(&d_diis, nvar * (2 + 2 * (size_t)m) + 1);
+        if (rc) { d_diis = nullptr; return rc; }
+        diis_m = m;
+        sfb::InstDesc I;
+        SFGPU_CUDA_TRY(cudaMemcpy(&I, d_inst, sizeof(I), cudaMemcpyDeviceToHost));
+        I.x = d_diis;
+        I.g = I.x + nvar;
+        I.XR = I.g + nvar;
+        I.XX0 = I.XR + nvar * (size_t)m;
+        SFGPU_CUDA_TRY(cudaMemcpy(d_inst_solve, &I, sizeof(I), cudaMemcpyHostToDevice));
+    }
+    double *err = d_diis + nvar * (2 + 2 * (size_t)diis_m);
+    SFGPU_CUDA_TRY(cudaMemcpyAsync(d_diis, x, sizeof(double) * nvar, cudaMemcpyHostToDevice, st));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(d_diis_int, 0, sizeof(int) * 4, st));
+    GroupShape sh = *group_shape_;
+    if (sh.dim == 1) group_shape(this, 2, 0, m, &sh);
+    const int rc = group_diis(sh, d_inst_solve, 1, 1, d_diis_int, m, eta, tol, maxit, d_diis_int + 1,
+                              d_diis_int + 2, err, st);
+    if (rc) return rc;
+    int v[2];
+    double e;
+    SFGPU_CUDA_TRY(cudaMemcpyAsync(x, d_diis, sizeof(double) * nvar, cudaMemcpyDeviceToHost, st));
+    SFGPU_CUDA_TRY(cudaMemcpyAsync(v, d_diis_int + 1, sizeof(v), cudaMemcpyDeviceToHost, st));
+    SFGPU_CUDA_TRY(cudaMemcpyAsync(&e, err, sizeof(e), cudaMemcpyDeviceToHost, st));
+    SFGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    if (iterations) *iterations = v[1];
+    if (final_error) *final_error = e;
+    return v[0];
 }
 
 // Overflow protection (sys : overflow_protection, SF_System.cpp:67, :445-519):
@@ -1232,6 +1398,7 @@ int sfgpu_system::set_orientation(int enable) {
 }
 
 int sfgpu_system::residual_async(const double *x, double *f) {
+    if (group_shape_) return group_residual(*group_shape_, d_inst, x, f, stream);
     const DLat &L = H.L;
     const int g = grid_for(M);
     cudaStream_t s = stream;
@@ -1493,6 +1660,8 @@ static int create_system(const sfgpu_system_desc *desc, int stride, sfgpu_system
     // the log-space chains (overflow protection) keep every slice
     s->primal_stride = desc->overflow_protection ? 0 : stride;
     int rc = s->setup(desc);
+    if (!rc) rc = s->setup_group();
+    if (!rc && s->group) rc = s->setup_group_single();
     if (rc) { delete s; return rc; }
     *out = s;
     return SFGPU_OK;

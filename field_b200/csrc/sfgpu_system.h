@@ -4,6 +4,9 @@
 #include "sfgpu_logspace.cuh"
 #include "sfgpu_charge.cuh"
 
+struct GroupShape;
+namespace sfb { struct InstDesc; }
+
 struct HostLat {
     DLat L;
     std::vector<double> lam_m, lam_p, lamc_m, lamc_p, Lx, w_gn, w_f;
@@ -152,6 +155,22 @@ struct sfgpu_system {
     sfk::QParam qp;
     double *d_neut_phib = nullptr, *d_el = nullptr, *d_surf = nullptr;
     int setup_charges(const sfgpu_system_desc *d, const std::vector<int> &jmap);
+    // the cluster engine (sfgpu_group.cuh), where it takes this system: its
+    // launch shape, the descriptor on the device and Pure_DIIS's vectors
+    // (x, g and m steps twice; allocated by the first solve, then kept)
+    bool group = false;
+    std::vector<int> jmap_h;
+    int *d_smap = nullptr, *d_jall = nullptr;
+    double *d_wpart = nullptr, *d_slices1 = nullptr;
+    GroupShape *group_shape_ = nullptr;
+    sfb::InstDesc *d_inst = nullptr, *d_inst_solve = nullptr;
+    double *d_diis = nullptr;
+    int diis_m = 0;
+    int *d_diis_int = nullptr;
+    int upload_chains(sfb::InstDesc *I);
+    int setup_group();
+    int setup_group_single();
+    int solve_group(double *x, double tol, int maxit, int m, double eta, int *iterations, double *final_error);
     std::vector<void *> allocs;
 
     ~sfgpu_system();
