@@ -70,9 +70,8 @@ __global__ void adj_dot_partial(int M, const double *__restrict__ a, const doubl
 // solvent) or theta / GN (restricted); the solvent's phibulk = 1 - others'
 __global__ void adj_mol_scalar(MolParam p, int nparts, const double *__restrict__ partial,
                                const MolScal *__restrict__ scal, AdjScal *__restrict__ as, int self) {
+    const double dot = sum_in_order(nparts, partial);   // sum phibar . phi
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double dot = 0;                      // sum phibar . phi
-    for (int b = 0; b < nparts; b++) dot += partial[b];
     const MolScal s = scal[self];
     AdjScal a = as[self];
     a.cbar = (s.norm != 0) ? dot / s.norm : 0.0;
@@ -121,9 +120,8 @@ __global__ void fe_zero_scal(int nmol, AdjScal *__restrict__ as) {
 }
 __global__ void fe_set_lncbar(int nparts, const double *__restrict__ partial, double invN, AdjScal *__restrict__ as,
                               int mol) {
+    const double v = sum_in_order(nparts, partial);
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double v = 0;
-    for (int b = 0; b < nparts; b++) v += partial[b];
     as[mol].lncbar = invN * v;
 }
 
@@ -131,12 +129,13 @@ __global__ void adj_qbar_scale(const AdjScal *__restrict__ as, int mol, double *
     if (threadIdx.x == 0 && blockIdx.x == 0) *out = as[mol].qbar;
 }
 
-// xbar(j, class) -= Gbar_full * G_full at the sites with iteration variables
+// xbar(j, class) -= Gbar_full * G_full + H at the sites with iteration variables
 struct SwfAdj {
     int nseg, nclass;
     int cls[SFGPU_MAX_SEG];
     int pinned[SFGPU_MAX_SEG];
     const double *gbar[SFGPU_MAX_SEG], *gfull[SFGPU_MAX_SEG], *range[SFGPU_MAX_SEG];
+    const double *h[SFGPU_MAX_SEG];   // Gbar . G collected as a product (adj_gather_*)
 };
 __global__ void adj_swf(int nsites, SwfAdj sa, const int *__restrict__ sites, double *__restrict__ xbar) {
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nsites; j += gridDim.x * blockDim.x) {
@@ -145,7 +144,7 @@ __global__ void adj_swf(int nsites, SwfAdj sa, const int *__restrict__ sites, do
             if (sa.cls[i] < 0) continue;
             double gb = sa.gbar[i][z];
             if (sa.pinned[i] && !(sa.range[i][z] > 0)) gb = 0;
-            xbar[(size_t)j * sa.nclass + sa.cls[i]] -= gb * sa.gfull[i][z];
+            xbar[(size_t)j * sa.nclass + sa.cls[i]] -= gb * sa.gfull[i][z] + sa.h[i][z];
         }
     }
 }
@@ -156,13 +155,16 @@ __global__ void adj_swf(int nsites, SwfAdj sa, const int *__restrict__ sites, do
 int sfgpu_system::ensure_adjoint_misc() {
     int rc;
     if (!a_misc) {
-        a_phibar.assign(nseg, nullptr); a_gbar.assign(nseg, nullptr); a_phibar_raw.assign(nseg, nullptr);
+        a_phibar.assign(nseg, nullptr); a_gbar.assign(nseg, nullptr); a_phibar_raw.assign(nseg, nullptr); a_h.assign(nseg, nullptr);
         for (int i = 0; i < nseg; i++) {
             if ((rc = alloc_d(&a_phibar[i], M)) || (rc = alloc_d(&a_gbar[i], M)) ||
-                (rc = alloc_d(&a_phibar_raw[i], M)))
+                (rc = alloc_d(&a_phibar_raw[i], M)) || (rc = alloc_d(&a_h[i], M)))
                 return rc;
         }
         if ((rc = alloc_d(&a_cot[0], (size_t)K * M)) || (rc = alloc_d(&a_cot[1], (size_t)K * M))) return rc;
+        // the gathering steps read surface layers, which no step writes
+        SFGPU_CUDA_TRY(cudaMemset(a_cot[0], 0, sizeof(double) * K * M));
+        SFGPU_CUDA_TRY(cudaMemset(a_cot[1], 0, sizeof(double) * K * M));
         if ((rc = alloc_d(&a_scal, sizeof(AdjScal) / sizeof(double) * (size_t)nmol)) || (rc = alloc_d(&a_chibbar, SFGPU_MAX_SEG)) ||
             (rc = alloc_d(&a_qbar, 1)))
             return rc;
@@ -459,7 +461,7 @@ int sfgpu_system::molecule_phi_store(int m) {
         MolParam p1 = p;
         p1.K = 1;   // a monomer's end distribution is G itself
         wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, d_gseg[i], d_wgn, d_partial);
-        mol_scalars<<<1, 1, 0, s>>>(p1, nblocks_red, d_partial, scal, m);
+        mol_scalars<<<1, 32, 0, s>>>(p1, nblocks_red, d_partial, scal, m);
         finalize_phi<<<g, kBlock, 0, s>>>(M, d_gseg[i], o.d_phi[i], scal, m, 1);
         return SFGPU_OK;
     }
@@ -468,7 +470,7 @@ int sfgpu_system::molecule_phi_store(int m) {
     int rc = store_chains(m, true, &gb0);
     if (rc) return rc;
     wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, K, gb0, d_wgn, d_partial);
-    mol_scalars<<<1, 1, 0, s>>>(p, nblocks_red, d_partial, scal, m);
+    mol_scalars<<<1, 32, 0, s>>>(p, nblocks_red, d_partial, scal, m);
     for (int i : o.used) {
         finalize_phi<<<g, kBlock, 0, s>>>(M, d_gseg[i], o.d_phi[i], scal, m, 0);
         set_boundaries<<<g, kBlock, 0, s>>>(L, 1, o.d_phi[i]);
@@ -513,7 +515,7 @@ int sfgpu_system::molecule_adjoint(int m, double *const *phibar_src) {
         int i = o.used[a];
         adj_dot_partial<<<np, kBlock, 0, s>>>(M, phibar_src[i], o.d_phi[i], d_partial + a * np);
     }
-    adj_mol_scalar<<<1, 1, 0, s>>>(p, np * (int)o.used.size(), d_partial, scal, as, m);
+    adj_mol_scalar<<<1, 32, 0, s>>>(p, np * (int)o.used.size(), d_partial, scal, as, m);
     for (int i : o.used)
         adj_phi_cd<<<g, kBlock, 0, s>>>(L, phibar_src[i], o.d_phi[i], d_gseg[i], scal, m, o.type == 0,
                                          a_phibar_raw[i], a_gbar[i]);
@@ -538,6 +540,36 @@ int sfgpu_system::molecule_adjoint(int m, double *const *phibar_src) {
     const size_t KM = (size_t)K * M;
     auto GF = [&](int j) -> const double * { return (a_stride ? a_bufF : a_gf) + (size_t)j * KM; };
     auto GB = [&](int j) -> const double * { return (a_stride ? a_bufB : a_gb) + (size_t)j * KM; };
+    if (K == 1 && o.force == 0 && !lat_twelve(L)) {
+        // gathering sweeps (adj_gather_*): cot and nxt hold y
+        const int XC = 8;   // planes a block marches through: as the composing primal step's
+        auto step = [&](int t, const double *y, const double *P, const double *Q, bool lngn) -> int {
+            const int sg = o.seg[t];
+            AdjStep a{y, a_phibar_raw[sg], P, d_gseg[sg], Q, lngn ? d_wgn : nullptr, a_qbar, a_h[sg], nxt};
+            cudaError_t e;
+            if (L.grad == 3) {
+                const dim3 grid((L.Md[2] - 2 + kTZ - 1) / kTZ, (L.Md[1] - 2 + kTY - 1) / kTY, (L.Md[0] - 2 + XC - 1) / XC);
+                e = y ? launch_pdl(adj_gather_march<false>, grid, dim3(kTZ * kTY), s, L, a, XC)
+                      : launch_pdl(adj_gather_march<true>, grid, dim3(kTZ * kTY), s, L, a, XC);
+            } else {
+                e = launch_pdl(adj_gather_rows, dim3(gr), dim3(kBlock), s, L, a);
+            }
+            std::swap(cot, nxt);
+            if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+            return rcs;
+        };
+        int rc = SFGPU_OK;
+        for (int t = N - 1; t >= 0 && !rc; t--) {      // forward recursion, descending
+            const int j = at(t);
+            rc = step(t, t == N - 1 ? nullptr : cot, GB(j), GF(j), false);
+        }
+        adj_qbar_scale<<<1, 1, 0, s>>>(as, m, a_qbar);
+        for (int t = 0; t < N && !rc; t++) {           // backward recursion, ascending
+            const int j = at(t);
+            rc = step(t, t == 0 ? nullptr : cot, GF(j), GB(j), t == 0);
+        }
+        return rc;
+    }
     // one reverse step: gbar(seg t) += cot . A p; nxt += A^T (G_t cot)
     auto rstep = [&](int t, const double *p, double S, int backward) {
         const int sg = o.seg[t];
@@ -751,6 +783,7 @@ int sfgpu_system::vjp_async(const double *x, const double *w, double *f, double 
     for (int i = 0; i < nseg; i++) {
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_phibar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_gbar[i], 0, sizeof(double) * M, s));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_h[i], 0, sizeof(double) * M, s));
     }
     SFGPU_CUDA_TRY(cudaMemsetAsync(a_chibbar, 0, sizeof(double) * SFGPU_MAX_SEG, s));
     SFGPU_CUDA_TRY(cudaMemsetAsync(xbar, 0, sizeof(double) * nvar, s));
@@ -783,6 +816,7 @@ int sfgpu_system::vjp_async(const double *x, const double *w, double *f, double 
         sa.cls[i] = class_of[i];
         sa.pinned[i] = freedom[i] == SFGPU_SEG_PINNED;
         sa.gbar[i] = a_gbar[i];
+        sa.h[i] = a_h[i];
         sa.gfull[i] = d_gfull[i];
         sa.range[i] = d_range[i];
     }
@@ -810,6 +844,7 @@ int sfgpu_system::free_energy_grad(const double *x, double *F, double *xbar) {
     for (int i = 0; i < nseg; i++) {
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_phibar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_gbar[i], 0, sizeof(double) * M, s));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_h[i], 0, sizeof(double) * M, s));
     }
     FeAdjParam fp;
     memset(&fp, 0, sizeof(fp));
@@ -823,7 +858,7 @@ int sfgpu_system::free_energy_grad(const double *x, double *F, double *xbar) {
         HMol &o = mols[m];
         for (size_t a = 0; a < o.used.size(); a++)
             adj_dot_partial<<<np, kBlock, 0, s>>>(M, d_wf, o.d_phi[o.used[a]], d_partial + a * np);
-        fe_set_lncbar<<<1, 1, 0, s>>>(np * (int)o.used.size(), d_partial, 1.0 / o.N, as, m);
+        fe_set_lncbar<<<1, 32, 0, s>>>(np * (int)o.used.size(), d_partial, 1.0 / o.N, as, m);
         for (int i : o.used) fe_gbar<<<g, kBlock, 0, s>>>(M, o.d_phi[i], d_wf, d_gseg[i], a_gbar[i]);
     }
     auto mol_adj = [&](int m) -> int {
@@ -854,6 +889,7 @@ int sfgpu_system::free_energy_grad(const double *x, double *F, double *xbar) {
         sa.cls[i] = class_of[i];
         sa.pinned[i] = freedom[i] == SFGPU_SEG_PINNED;
         sa.gbar[i] = a_gbar[i];
+        sa.h[i] = a_h[i];
         sa.gfull[i] = d_gfull[i];
         sa.range[i] = d_range[i];
     }
@@ -872,6 +908,7 @@ int sfgpu_system::phi_vjp_async(const double *x, const double *const *omega, dou
     for (int i = 0; i < nseg; i++) {
         SFGPU_CUDA_TRY(cudaMemcpyAsync(a_phibar[i], omega[i], sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_gbar[i], 0, sizeof(double) * M, s));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_h[i], 0, sizeof(double) * M, s));
     }
     fe_zero_scal<<<1, 1, 0, s>>>(nmol, (AdjScal *)a_scal);
     int held = (mols[solvent].type != 0 && !mols[solvent].ring && !mols[solvent].tree && !mols[solvent].dend) ? solvent : -1;
@@ -895,6 +932,7 @@ int sfgpu_system::phi_vjp_async(const double *x, const double *const *omega, dou
         sa.cls[i] = class_of[i];
         sa.pinned[i] = freedom[i] == SFGPU_SEG_PINNED;
         sa.gbar[i] = a_gbar[i];
+        sa.h[i] = a_h[i];
         sa.gfull[i] = d_gfull[i];
         sa.range[i] = d_range[i];
     }

@@ -4,8 +4,9 @@
 // with Gf(s) = G_s * A Gf(s-1) and Gb(s) = G_s * A Gb(s+1),
 //   Fbar(s-1) = phibar_raw . Gb(s-1) + A^T (G_s * Fbar(s)),   Gbar_s += Fbar(s) * A Gf(s-1)
 //   Bbar(s+1) = phibar_raw . Gf(s+1) + A^T (G_s * Bbar(s)),   Gbar_s += Bbar(s) * A Gb(s+1)
-// run as a descending and an ascending sweep over stored Gf and Gb.  A^T is
-// applied by scattering every interior value to the (mapped) sites its
+// run as a descending and an ascending sweep over stored Gf and Gb.  On the
+// 1D, 2D and six-neighbour 3D lattices A^T is gathered (adj_gather_*); the
+// other steps scatter every interior value to the (mapped) sites their
 // stencil reads, with FP64 atomics.
 #pragma once
 #include "sfgpu_tangent.cuh"
@@ -157,6 +158,168 @@ static __global__ void adj_chain_step(DLat L, const double *__restrict__ cot, co
         gbar[t] += c * raw1_row(L, R, p, k, nlast);
         scatter1(L, R, k, nlast, G[t] * c, out);
     });
+}
+
+// ---- reverse chain steps by gathering --------------------------------------
+// With c_t the cotangent of the propagator at position t and y_t = G_t c_t,
+// one step of either sweep is
+//   c' = phibar_raw' . P' + A^T y,   H' += c' Q',   y' = G' c',
+// primes at the position stepped to, P' the other sweep's stored slice there
+// (Gb descending, Gf ascending) and Q' this sweep's own.  H collects
+// Gbar . G directly: every step has the factor G, so c_t . A p = c_t Q_t / G_t
+// and the stencil of the stored slice is never formed again.  A^T is gathered:
+// on the six-neighbour and 1D/2D lattices the readers of a site are its
+// neighbours, with the weights below where a boundary maps a read back inside.
+//
+// Bound by memory: y, P', phibar_raw', G', Q', H' read, y', H' written, 64 B a
+// site and step.  The scatter it replaces took 6 FP64 atomics a site, a pass
+// of its own for phibar_raw . P and the stencil of the slice: 46 + 9 us a step
+// on a 128^3 lattice, 26 now.
+
+// weight with which A^T at coordinate s of gradient d takes the lower / upper
+// neighbour (index lat_mapc of s -+ 1), for a step of weight 1 to either side
+__device__ __forceinline__ double gather_lo(const DLat &L, int d, int s) {
+    const int bc = L.bc_lo[d];
+    if (s == 1) return (bc == SFGPU_BOUND_MIRROR2 || bc == SFGPU_BOUND_SURFACE) ? 0.0 : 1.0;
+    return (s == 2 && bc == SFGPU_BOUND_MIRROR2) ? 2.0 : 1.0;
+}
+__device__ __forceinline__ double gather_hi(const DLat &L, int d, int s) {
+    const int bc = L.bc_hi[d], n = L.Md[d] - 2;
+    if (s == n) return (bc == SFGPU_BOUND_MIRROR2 || bc == SFGPU_BOUND_SURFACE) ? 0.0 : 1.0;
+    return (s == n - 1 && bc == SFGPU_BOUND_MIRROR2) ? 2.0 : 1.0;
+}
+// the same along a radial gradient, whose readers step with lambda-+ of their own layer
+__device__ __forceinline__ double gather_lo_curved(const DLat &L, int s) {
+    const int bc = L.bc_lo[0], n = L.Md[0] - 2;
+    if (s == 1) return bc == SFGPU_BOUND_MIRROR1 ? L.lam_m[1] : bc == SFGPU_BOUND_PERIODIC ? L.lam_p[n] : 0.0;
+    return L.lam_p[s - 1] + ((s == 2 && bc == SFGPU_BOUND_MIRROR2) ? L.lam_m[1] : 0.0);
+}
+__device__ __forceinline__ double gather_hi_curved(const DLat &L, int s) {
+    const int bc = L.bc_hi[0], n = L.Md[0] - 2;
+    if (s == n) return bc == SFGPU_BOUND_MIRROR1 ? L.lam_p[n] : bc == SFGPU_BOUND_PERIODIC ? L.lam_m[1] : 0.0;
+    return L.lam_m[s + 1] + ((s == n - 1 && bc == SFGPU_BOUND_MIRROR2) ? L.lam_p[n] : 0.0);
+}
+// (A^T y) at interior position k of row R of a 1D or 2D lattice
+__device__ __forceinline__ double gather1_row(const DLat &L, const RowInfo &R, const double *__restrict__ y, int k,
+                                              int nlast) {
+    const int d = L.grad - 1;
+    const int t = R.base + k;
+    const double a = y[R.base + ((k == 1) ? L.map_lo[d] : k - 1)], c = y[R.base + ((k == nlast) ? L.map_hi[d] : k + 1)];
+    const double b = y[t];
+    if (L.grad == 1) {
+        if (L.cyl) return (1.0 - L.lam_m[k] - L.lam_p[k]) * b + gather_lo_curved(L, k) * a + gather_hi_curved(L, k) * c;
+        return (1.0 - 2.0 * L.l1) * b + L.l1 * (gather_lo(L, 0, k) * a + gather_hi(L, 0, k) * c);
+    }
+    const double u = y[t + R.up], dn = y[t + R.dn];
+    const double row = L.l1 * (gather_lo(L, 1, k) * a + gather_hi(L, 1, k) * c);
+    if (L.cyl)
+        return (1.0 - L.lam_m[R.x] - L.lam_p[R.x] - 2.0 * L.l1) * b + gather_lo_curved(L, R.x) * u +
+               gather_hi_curved(L, R.x) * dn + row;
+    return (1.0 - 4.0 * L.l1) * b + L.l1 * (gather_lo(L, 0, R.x) * u + gather_hi(L, 0, R.x) * dn) + row;
+}
+
+// operands of one reverse step; y == nullptr starts a sweep (no A^T y), w the
+// lnGN weights whose cotangent *qbar enters the first ascending one
+struct AdjStep {
+    const double *y, *pr, *P, *G, *Q, *w, *qbar;
+    double *H, *out;
+};
+static __global__ void adj_gather_rows(DLat L, AdjStep a) {
+    sfk::pdl_enter();
+    const int worker = blockIdx.x * blockDim.x + threadIdx.x;
+    for_interior(L, worker, gridDim.x * blockDim.x, [&](const RowInfo &R, int k, int nlast) {
+        const int t = R.base + k;
+        double c = a.pr[t] * a.P[t];
+        if (a.w) c += *a.qbar * a.w[t];
+        if (a.y) c += gather1_row(L, R, a.y, k, nlast);
+        a.H[t] += c * a.Q[t];
+        a.out[t] = a.G[t] * c;
+    });
+}
+
+// the same on the six-neighbour 3D lattices, marching through x as
+// step3d_march_pf does (a 32 x 8 tile of columns, plane x + 1's loads in
+// flight while plane x is computed)
+template <bool kStart>
+static __global__ void __launch_bounds__(kTZ * kTY, 3) adj_gather_march(DLat L, AdjStep o, int xc) {
+    __shared__ double tile[2][kTY + 2][kTZ + 2];
+    sfk::pdl_enter();
+    const int nx = L.Md[0] - 2, ny = L.Md[1] - 2, nz = L.Md[2] - 2;
+    const int jx = L.st[0], jy = L.st[1];
+    const int tz = threadIdx.x % kTZ, ty = threadIdx.x / kTZ;
+    const int z = blockIdx.x * kTZ + tz + 1;
+    const int y = blockIdx.y * kTY + ty + 1;
+    const int x0 = blockIdx.z * xc + 1;
+    if (x0 > nx) return;
+    const int x1 = min(x0 + xc - 1, nx);
+    const bool act = (z <= nz) && (y <= ny);
+    const int zm = lat_mapc(L, 2, z - 1), zp = lat_mapc(L, 2, z + 1);
+    const int ym = lat_mapc(L, 1, y - 1), yp = lat_mapc(L, 1, y + 1);
+    const bool hz0 = (tz == 0), hz1 = (tz == kTZ - 1) || (z == nz);
+    const bool hy0 = (ty == 0), hy1 = (ty == kTY - 1) || (y == ny);
+    const int col = y * jy + z;
+    const double wzl = act ? gather_lo(L, 2, z) * (1.0 / 6.0) : 0.0, wzh = act ? gather_hi(L, 2, z) * (1.0 / 6.0) : 0.0;
+    const double wyl = act ? gather_lo(L, 1, y) * (1.0 / 6.0) : 0.0, wyh = act ? gather_hi(L, 1, y) * (1.0 / 6.0) : 0.0;
+    double vprev = 0, vcur = 0, vnext = 0, hzl = 0, hzh = 0, hyl = 0, hyh = 0, g = 0, pr = 0, P = 0, Q = 0, H = 0;
+    auto load = [&](int x, double &g_, double &pr_, double &P_, double &Q_, double &H_) {
+        const int t = x * jx + col;
+        g_ = o.G[t]; pr_ = o.pr[t]; P_ = o.P[t]; Q_ = o.Q[t]; H_ = o.H[t];
+    };
+    auto halos = [&](int x, double &a, double &b, double &c, double &d) {
+        const int base = x * jx;
+        if (hz0) a = o.y[base + y * jy + zm];
+        if (hz1) b = o.y[base + y * jy + zp];
+        if (hy0) c = o.y[base + ym * jy + z];
+        if (hy1) d = o.y[base + yp * jy + z];
+    };
+    if (act) {
+        load(x0, g, pr, P, Q, H);
+        if (!kStart) {
+            vprev = o.y[lat_mapc(L, 0, x0 - 1) * jx + col];
+            vcur = o.y[x0 * jx + col];
+            vnext = o.y[lat_mapc(L, 0, x0 + 1) * jx + col];
+            halos(x0, hzl, hzh, hyl, hyh);
+        }
+    }
+    const double qb = (kStart && o.w) ? *o.qbar : 0.0;
+    int b = 0;
+    for (int x = x0; x <= x1; x++) {
+        double vn2 = 0, nzl = 0, nzh = 0, nyl = 0, nyh = 0, gn = 0, prn = 0, Pn = 0, Qn = 0, Hn = 0;
+        if (act && x < x1) {
+            load(x + 1, gn, prn, Pn, Qn, Hn);
+            if (!kStart) {
+                vn2 = o.y[lat_mapc(L, 0, x + 2) * jx + col];
+                halos(x + 1, nzl, nzh, nyl, nyh);
+            }
+        }
+        if (!kStart) {
+            if (act) {
+                tile[b][ty + 1][tz + 1] = vcur;
+                if (hz0) tile[b][ty + 1][0] = hzl;
+                if (hz1) tile[b][ty + 1][tz + 2] = hzh;
+                if (hy0) tile[b][0][tz + 1] = hyl;
+                if (hy1) tile[b][ty + 2][tz + 1] = hyh;
+            }
+            __syncthreads();
+        }
+        if (act) {
+            const int t = x * jx + col;
+            double c = pr * P;
+            if (kStart) {
+                if (o.w) c += qb * o.w[t];
+            } else {
+                c += (gather_lo(L, 0, x) * vprev + gather_hi(L, 0, x) * vnext) * (1.0 / 6.0);
+                c += wyl * tile[b][ty][tz + 1] + wyh * tile[b][ty + 2][tz + 1];
+                c += wzl * tile[b][ty + 1][tz] + wzh * tile[b][ty + 1][tz + 2];
+            }
+            o.H[t] = H + c * Q;
+            o.out[t] = g * c;
+        }
+        vprev = vcur; vcur = vnext; vnext = vn2;
+        hzl = nzl; hzh = nzh; hyl = nyl; hyh = nyh;
+        g = gn; pr = prn; P = Pn; Q = Qn; H = Hn;
+        b ^= 1;
+    }
 }
 
 // out[k][t] = phibar_raw[t] * q[k][t] on interior sites (0 elsewhere), K components
@@ -540,6 +703,9 @@ __device__ __forceinline__ void side_scatter(const DLat &L, int z, double y, dou
 
 static __global__ void adj_residual(DLat L, ResParam rp, ChiTable ct, const int *__restrict__ sites,
                                     const double *__restrict__ w, AdjResParam ap, double *__restrict__ xbar) {
+    double chib[SFGPU_MAX_SEG];          // this thread's part of every class's chibbar
+#pragma unroll
+    for (int c = 0; c < SFGPU_MAX_SEG; c++) chib[c] = 0;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < rp.nsites; j += gridDim.x * blockDim.x) {
         const int z = sites[j];
         double phit = 0;
@@ -568,12 +734,31 @@ static __global__ void adj_residual(DLat L, ResParam rp, ChiTable ct, const int 
             }
             phitbar += ub[c] * ci / (phit * phit);
             xbar[(size_t)j * rp.nclass + c] += ub[c];     // u' contains -ln G = x
-            atomicAdd(ap.chibbar + c, ub[c]);
         }
+#pragma unroll
+        for (int c = 0; c < SFGPU_MAX_SEG; c++)
+            if (c < rp.nclass) chib[c] += ub[c];
         for (int i = 0; i < rp.nseg; i++) {
             atomicAdd(ap.phibar[i] + z, phitbar);
             if (rhobar[i] != 0) side_scatter(L, z, rhobar[i], ap.phibar[i]);
         }
+    }
+    // one addition per block and class (one per site made every site of the
+    // lattice wait at the same few addresses: 6.7 ms on 128^3, 0.25 now)
+    __shared__ double red[kBlock / 32];
+#pragma unroll
+    for (int c = 0; c < SFGPU_MAX_SEG; c++) {
+        if (c >= rp.nclass) break;
+        double v = chib[c];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            v = 0;
+            for (int w = 0; w < kBlock / 32; w++) v += red[w];
+            atomicAdd(ap.chibbar + c, v);
+        }
+        __syncthreads();
     }
 }
 

@@ -21,6 +21,44 @@ __device__ __forceinline__ void pdl_enter() {
 
 constexpr int kBlock = 256;
 
+// p[0] + p[1] + ... in this order, by one full warp (of at
+// most four in the block): the lanes bring 256 values
+// at a time, lane 0 (whose result counts) adds them.  One thread alone waits
+// for a load per addition: 96 us for the 2368 partial sums of a 128^3 lattice,
+// 14 this way.
+__device__ __forceinline__ double sum_in_order(int n, const double *__restrict__ p) {
+    __shared__ double buf[4][256];
+    const int lane = threadIdx.x & 31;
+    double *w = buf[(threadIdx.x >> 5) & 3];
+    double v = 0, e[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) e[u] = (32 * u + lane < n) ? p[32 * u + lane] : 0.0;
+    for (int b = 0; b < n; b += 256) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) w[32 * u + lane] = e[u];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = b + 256 + 32 * u + lane;
+            e[u] = (i < n) ? p[i] : 0.0;
+        }
+        if (lane == 0) {
+            const int k = min(256, n - b);
+            int i = 0;
+            for (; i + 16 <= k; i += 16) {
+                double q[16];
+#pragma unroll
+                for (int u = 0; u < 16; u++) q[u] = w[i + u];
+#pragma unroll
+                for (int u = 0; u < 16; u++) v += q[u];
+            }
+            for (; i < k; i++) v += w[i];
+        }
+        __syncwarp();
+    }
+    return v;
+}
+
 struct MolScal {            // per-molecule device scalars
     double lngn, phibulk, lnc, norm;
 };
@@ -810,9 +848,8 @@ struct MolParam {
 };
 static __global__ void mol_scalars(MolParam p, int nblocks, const double *__restrict__ partial,
                             MolScal *__restrict__ scal, int self) {
+    double v = sum_in_order(nblocks, partial);
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double v = 0;
-    for (int b = 0; b < nblocks; b++) v += partial[b];
     if (p.K > 1) v /= 6.0;   // six bond directions (lumped or not)
     MolScal s;
     s.lngn = log(v);
@@ -1317,11 +1354,10 @@ static __global__ void dots_partial(size_t len, DotList dl, double *__restrict__
 }
 
 static __global__ void finish_sums(int n, int nblocks, const double *__restrict__ partial, double *__restrict__ out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double acc = 0;
-    for (int b = 0; b < nblocks; b++) acc += partial[(size_t)i * nblocks + b];
-    out[i] = acc;
+    for (int i = threadIdx.x >> 5; i < n; i += blockDim.x >> 5) {
+        const double acc = sum_in_order(nblocks, partial + (size_t)i * nblocks);
+        if ((threadIdx.x & 31) == 0) out[i] = acc;
+    }
 }
 
 // DIIS step pieces (SFNewton::PlainLBFGSDIIS, sfnewton.cpp:602-661)

@@ -44,23 +44,6 @@ static int grid_rows(const DLat &L) {
     return (int)std::max(1L, std::min(b, 148L * 32));
 }
 
-// a step launch with programmatic stream serialization: the kernel may be
-// scheduled while the previous one drains and waits for it in pdl_enter()
-template <class... KArgs, class... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // first-order step inside a residual evaluation: x-marching tiles on the
 // six-neighbour 3D lattices (launched as programmatic dependents of the
 // step before), row-wise otherwise
@@ -1077,7 +1060,7 @@ int sfgpu_system::molecule_phi_dend(int m) {
     p.pinned = o.pinned; p.solvent = (m == solvent); p.nmol = nmol;
     p.phibulk_in = o.phibulk; p.theta = o.theta;
     wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, cur, d_wgn, d_partial);
-    mol_scalars<<<1, 1, 0, s>>>(p, nblocks_red, d_partial, (MolScal *)d_scal, m);
+    mol_scalars<<<1, 32, 0, s>>>(p, nblocks_red, d_partial, (MolScal *)d_scal, m);
     for (int i : o.used) {
         finalize_phi<<<g, kBlock, 0, s>>>(M, d_gseg[i], o.d_phi[i], (const MolScal *)d_scal, m, 0);
         set_boundaries<<<g, kBlock, 0, s>>>(L, 1, o.d_phi[i]);
@@ -1200,7 +1183,7 @@ int sfgpu_system::molecule_phi_tree(int m) {
     p.pinned = o.pinned; p.solvent = (m == solvent); p.nmol = nmol;
     p.phibulk_in = o.phibulk; p.theta = o.theta;
     wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, U(0), d_wgn, d_partial);
-    mol_scalars<<<1, 1, 0, s>>>(p, nblocks_red, d_partial, (MolScal *)d_scal, m);
+    mol_scalars<<<1, 32, 0, s>>>(p, nblocks_red, d_partial, (MolScal *)d_scal, m);
     for (int i : o.used) {
         finalize_phi<<<g, kBlock, 0, s>>>(M, d_gseg[i], o.d_phi[i], (const MolScal *)d_scal, m, 0);
         set_boundaries<<<g, kBlock, 0, s>>>(L, 1, o.d_phi[i]);
@@ -1249,7 +1232,7 @@ int sfgpu_system::molecule_phi(int m) {
         // lnGN of the end-point distribution G itself (all K components equal)
         wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, d_gseg[i], d_wgn, d_partial);
         MolParam p1 = p; p1.K = 1;
-        mol_scalars<<<1, 1, 0, s>>>(p1, nblocks_red, d_partial, scal, m);
+        mol_scalars<<<1, 32, 0, s>>>(p1, nblocks_red, d_partial, scal, m);
         finalize_phi<<<g, kBlock, 0, s>>>(M, d_gseg[i], o.d_phi[i], scal, m, 1);
         return SFGPU_OK;
     }
@@ -1274,7 +1257,7 @@ int sfgpu_system::molecule_phi(int m) {
             cur = ginv; std::swap(ginv, tmp);
         }
         wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, cur, d_wgn, d_partial);
-        mol_scalars<<<1, 1, 0, s>>>(p, nblocks_red, d_partial, scal, m);
+        mol_scalars<<<1, 32, 0, s>>>(p, nblocks_red, d_partial, scal, m);
         finalize_phi<<<g, kBlock, 0, s>>>(M, G, phi, scal, m, 0);
         set_boundaries<<<g, kBlock, 0, s>>>(L, 1, phi);
         return SFGPU_OK;
@@ -1363,7 +1346,7 @@ int sfgpu_system::molecule_phi(int m) {
         cur = ginv; std::swap(ginv, tmp);
     }
     wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, K, cur, d_wgn, d_partial);
-    mol_scalars<<<1, 1, 0, s>>>(p, nblocks_red, d_partial, scal, m);
+    mol_scalars<<<1, 32, 0, s>>>(p, nblocks_red, d_partial, scal, m);
     for (int i : o.used) {
         finalize_phi<<<g, kBlock, 0, s>>>(M, d_gseg[i], o.d_phi[i], scal, m, 0);
         set_boundaries<<<g, kBlock, 0, s>>>(L, 1, o.d_phi[i]);

@@ -4,6 +4,23 @@
 #include "sfgpu_logspace.cuh"
 #include "sfgpu_charge.cuh"
 
+// a step launch with programmatic stream serialization: the kernel may be
+// scheduled while the previous one drains and waits for it in pdl_enter()
+template <class... KArgs, class... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 struct GroupShape;
 namespace sfb { struct InstDesc; }
 
@@ -114,7 +131,7 @@ struct sfgpu_system {
     void dend_view(HMol &o, bool on);
     double *a_ckF = nullptr, *a_ckB = nullptr, *a_bufF = nullptr, *a_bufB = nullptr;
     int a_qseg = -1;                        // segment held in a_bufF / a_bufB
-    std::vector<double *> a_phibar, a_gbar, a_phibar_raw;
+    std::vector<double *> a_phibar, a_gbar, a_phibar_raw, a_h;
     double *a_scal = nullptr, *a_chibbar = nullptr, *a_qbar = nullptr, *a_w = nullptr, *a_xbar = nullptr;
     int ensure_adjoint();
     int ensure_adjoint_misc();

@@ -99,8 +99,8 @@ int sfgpu_system::molecule_phi_t(int m) {
         MolParam p1 = p; p1.K = 1;
         wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, d_gseg[i], d_wgn, d_partial);
         wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, dgseg[i], d_wgn, d_dpartial);
-        mol_scalars<<<1, 1, 0, s>>>(p1, nblocks_red, d_partial, scal, m);
-        mol_scalars_t<<<1, 1, 0, s>>>(p1, nblocks_red, d_dpartial, scal, tscal, m);
+        mol_scalars<<<1, 32, 0, s>>>(p1, nblocks_red, d_partial, scal, m);
+        mol_scalars_t<<<1, 32, 0, s>>>(p1, nblocks_red, d_dpartial, scal, tscal, m);
         finalize_phi_t<<<g, kBlock, 0, s>>>(M, d_gseg[i], dgseg[i], o.d_phi[i], o.d_dphi[i], scal, tscal, m, 1);
         return SFGPU_OK;
     }
@@ -293,8 +293,8 @@ int sfgpu_system::molecule_phi_t(int m) {
     }
     wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, K, cur, d_wgn, d_partial);
     wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, K, dcur, d_wgn, d_dpartial);
-    mol_scalars<<<1, 1, 0, s>>>(p, nblocks_red, d_partial, scal, m);
-    mol_scalars_t<<<1, 1, 0, s>>>(p, nblocks_red, d_dpartial, scal, tscal, m);
+    mol_scalars<<<1, 32, 0, s>>>(p, nblocks_red, d_partial, scal, m);
+    mol_scalars_t<<<1, 32, 0, s>>>(p, nblocks_red, d_dpartial, scal, tscal, m);
     for (int i : o.used) {
         finalize_phi_t<<<g, kBlock, 0, s>>>(M, d_gseg[i], dgseg[i], o.d_phi[i], o.d_dphi[i], scal, tscal, m, 0);
         set_boundaries<<<g, kBlock, 0, s>>>(L, 1, o.d_phi[i]);

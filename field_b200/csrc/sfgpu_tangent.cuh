@@ -329,9 +329,8 @@ static __global__ void connect_t(int M, int K, const double *__restrict__ a, con
 // tangents of lnGN, phibulk and the normalisation (after mol_scalars ran)
 static __global__ void mol_scalars_t(MolParam p, int nblocks, const double *__restrict__ dpartial,
                                      const MolScal *__restrict__ scal, MolScalT *__restrict__ tscal, int self) {
+    double dv = sum_in_order(nblocks, dpartial);
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double dv = 0;
-    for (int b = 0; b < nblocks; b++) dv += dpartial[b];
     if (p.K > 1) dv /= 6.0;   // six bond directions, lumped or not (as mol_scalars)
     const MolScal s = scal[self];
     MolScalT t;
