@@ -318,8 +318,7 @@ void sfgpu_system::adj_fstep(const HMol &o, int t, const double *src, double *ds
         step2_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst,
                                                           nullptr, nullptr, COMP_NONE, 0);
     else
-        step2l_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst,
-                                                           nullptr, nullptr, COMP_NONE, 0);
+        launch_step2l(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
 }
 void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *dst, const double *other,
                              double *phi) {
@@ -340,8 +339,7 @@ void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *ds
         step2_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst,
                                                           other, phi, mode, 1);
     else
-        step2l_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst,
-                                                           other, phi, mode, 1);
+        launch_step2l(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
 }
 
 // Gf and Gb of every position of molecule m's chain (full chains, also for

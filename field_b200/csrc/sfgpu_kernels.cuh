@@ -757,6 +757,147 @@ static __global__ void step2l_rows(DLat L, const double *__restrict__ gin, const
     });
 }
 
+// The same step with the lattice's direction count and geometry fixed at
+// compile time (K = 3: 1D, K = 5: 2D) and one thread per site, a warp along
+// the last gradient.  Loops over components unroll, so outputs and weights
+// stay in registers and every load is issued before the first sum; same
+// operands, weights and summation order, bit-identical.  For 0 < S < 1, where
+// no weight but the opposite direction's is 0 (lump2_w); step2l_rows takes the
+// two end points.  The lattices are small and a step is latency: 61 x 77, K = 5
+// took 23 us with run-time component loops in local memory and a warp per row,
+// 3.2 us this way.
+template <int K>
+__device__ __forceinline__ constexpr int lump_axis(int k) {
+    return K == 3 ? (k == 1 ? -1 : 0) : (k == 2 ? -1 : (k == 0 || k == 4) ? 0 : 1);
+}
+template <int K>
+__device__ __forceinline__ constexpr int lump_sgn(int k) {
+    return K == 3 ? 1 - k : (k < 2 ? 1 : k == 2 ? 0 : -1);
+}
+template <int K>
+__device__ __forceinline__ constexpr int lump_opp(int k) { return K - 1 - k; }   // k itself for the lumped one
+template <int K>
+__device__ __forceinline__ constexpr double lump_mult(int k) { return K == 3 ? (k == 1 ? 4.0 : 1.0) : (k == 2 ? 2.0 : 1.0); }
+template <int K>
+__device__ __forceinline__ double lump_w(int kk, int kp, double S, double Lw) {
+    if (kk == kp) return (K == 3 && kk == 1) ? S + 2 * Lw : S;
+    return lump_mult<K>(kp) * Lw;
+}
+
+template <int K, bool kCyl>
+static __global__ void __launch_bounds__(128)
+step2l_sites(DLat L, const double *__restrict__ gin, const double *__restrict__ G, double S,
+             double *__restrict__ gout, const double *__restrict__ other, double *__restrict__ phi, int mode,
+             int backward) {
+    pdl_enter();
+    const int M = L.M;
+    const double Lw = (1.0 - S) / 4.0;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;                      // along the last gradient
+    const int row = (K == 5) ? blockIdx.y * blockDim.y + threadIdx.y + 1 : 0;     // along the first
+    const int x = (K == 5) ? row : k, y = (K == 5) ? k : 0;
+    const int nx = L.Md[0] - 2, ny = (K == 5) ? L.Md[1] - 2 : 0;
+    if (x > nx || (K == 5 && y > ny)) return;
+    const int t = (K == 5) ? x * L.st[0] + y : x;
+    // site and swap mode of a read one step along axis a, by sign
+    auto site = [&](int a, int d, int &sm) { return lump2_nb(L, x, y, a, d, sm); };
+    // the component read for kp across a boundary of axis a (lump2_read)
+    auto comp = [&](int kp, int a, int sm) {
+        if (lump_axis<K>(kp) != a) return kp;
+        return (sm == 1 || (sm == 2 && lump_sgn<K>(kp) > 0)) ? lump_opp<K>(kp) : kp;
+    };
+    const double g = G[t];
+    double oth[K], ph = 0;
+#pragma unroll
+    for (int c = 0; c < K; c++) oth[c] = 0;
+    if (mode == COMP_ACC) {
+        ph = phi[t];
+#pragma unroll
+        for (int c = 0; c < K; c++) oth[c] = other[(size_t)c * M + t];
+    }
+    double fm = 0, fp = 0, own[K];
+    if (kCyl) {
+        fm = 6 * L.lam_m[x];
+        fp = 6 * L.lam_p[x];
+#pragma unroll
+        for (int c = 0; c < K; c++) own[c] = gin[(size_t)c * M + t];
+    }
+    double out[K];
+    if (!backward) {
+        double r[K][K];
+#pragma unroll
+        for (int kk = 0; kk < K; kk++) {
+            int sm = 0;
+            const int src = (lump_axis<K>(kk) >= 0) ? site(lump_axis<K>(kk), -lump_sgn<K>(kk), sm) : t;
+#pragma unroll
+            for (int kp = 0; kp < K; kp++) {
+                if (kp == lump_opp<K>(kk) && kp != kk) continue;
+                const int c = (lump_axis<K>(kk) >= 0) ? comp(kp, lump_axis<K>(kk), sm) : kp;
+                r[kk][kp] = gin[(size_t)c * M + src];
+            }
+        }
+#pragma unroll
+        for (int kk = 0; kk < K; kk++) {
+            double acc = 0;
+            bool first = true;
+#pragma unroll
+            for (int kp = 0; kp < K; kp++) {
+                if (kp == lump_opp<K>(kk) && kp != kk) continue;
+                double v = r[kk][kp];
+                if (kCyl && lump_axis<K>(kk) == 0) {
+                    // the mixture of a radial read with the reflected component (lump2_mix)
+                    const double f = (lump_sgn<K>(kk) < 0) ? fp : fm, fc = 1.0 - f;
+                    const int refl = (lump_axis<K>(kp) == 0) ? lump_opp<K>(kp) : kp;
+                    v = f * v + fc * own[refl];
+                }
+                v = lump_w<K>(kk, kp, S, Lw) * v;
+                acc = first ? v : acc + v;
+                first = false;
+            }
+            out[kk] = acc * g;
+        }
+    } else {
+        double v[K];
+#pragma unroll
+        for (int kp = 0; kp < K; kp++) {
+            int sm = 0;
+            const int src = (lump_axis<K>(kp) >= 0) ? site(lump_axis<K>(kp), lump_sgn<K>(kp), sm) : t;
+            const int c = (lump_axis<K>(kp) >= 0) ? comp(kp, lump_axis<K>(kp), sm) : kp;
+            v[kp] = gin[(size_t)c * M + src];
+        }
+        if (kCyl) {
+#pragma unroll
+            for (int kp = 0; kp < K; kp++) {
+                if (lump_axis<K>(kp) != 0 || !(K == 3 || lump_sgn<K>(kp) < 0)) continue;
+                const double f = (lump_sgn<K>(kp) > 0) ? fp : fm, fc = 1.0 - f;
+                v[kp] = f * v[kp] + fc * own[lump_opp<K>(kp)];
+            }
+        }
+#pragma unroll
+        for (int kq = 0; kq < K; kq++) {
+            double acc = 0;
+            bool first = true;
+#pragma unroll
+            for (int kp = 0; kp < K; kp++) {
+                if (kp == lump_opp<K>(kq) && kp != kq) continue;
+                const double u = lump_w<K>(kq, kp, S, Lw) * v[kp];
+                acc = first ? u : acc + u;
+                first = false;
+            }
+            out[kq] = acc * g;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < K; c++) gout[(size_t)c * M + t] = out[c];
+    if (mode == COMP_ACC) {
+#pragma unroll
+        for (int c = 0; c < K; c++) {
+            const double a = out[c] * oth[c];
+            ph += (lump_mult<K>(c) == 1.0) ? a : a * lump_mult<K>(c);
+        }
+        phi[t] = ph;
+    }
+}
+
 // multiplicity of direction component k of a K-component slice
 __host__ __device__ inline double comp_mult(int K, int k) {
     if (K == 3 && k == 1) return 4.0;

@@ -75,6 +75,28 @@ int sfgpu_system::launch_step1(const double *gin, const double *G, double *gout,
     return SFGPU_OK;
 }
 
+// lumped second-order step: step2l_sites, except at S = 0 or 1, where a weight
+// vanishes that it takes as nonzero
+int sfgpu_system::launch_step2l(const double *gin, const double *G, double S, double *gout, const double *other,
+                                double *phi, int mode, int backward) {
+    const DLat &L = H.L;
+    cudaError_t e;
+    if (S == 0.0 || S == 1.0) {
+        step2l_rows<<<grid_rows(L), kBlock, 0, stream>>>(L, gin, G, S, gout, other, phi, mode, backward);
+        e = cudaGetLastError();
+    } else if (L.grad == 1) {
+        const dim3 grid((L.Md[0] - 2 + 127) / 128);
+        e = launch_pdl(L.cyl ? step2l_sites<3, true> : step2l_sites<3, false>, grid, dim3(128), stream, L, gin, G, S, gout,
+                       other, phi, mode, backward);
+    } else {
+        const dim3 grid((L.Md[1] - 2 + 31) / 32, (L.Md[0] - 2 + 3) / 4);
+        e = launch_pdl(L.cyl ? step2l_sites<5, true> : step2l_sites<5, false>, grid, dim3(32, 4), stream, L, gin, G, S,
+                       gout, other, phi, mode, backward);
+    }
+    if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+    return SFGPU_OK;
+}
+
 // ---------------------------------------------------------------------------
 // lattice set-up (Lat1DFlat.cpp:4-149, Lat2DFlat.cpp:35-220,
 // Lat2DCylinder.cpp:7-55, Lat3D.cpp:44-236)
@@ -1285,8 +1307,7 @@ int sfgpu_system::molecule_phi(int m) {
                        pf[o.seg[t - 1] * nseg + sg], out, (const double *)nullptr, (double *)nullptr, (int)COMP_NONE, 0,
                        (int)STEP2_PLAIN);
         else
-            step2l_rows<<<grid_rows(L), kBlock, 0, s>>>(L, in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out,
-                                        nullptr, nullptr, COMP_NONE, 0);
+            launch_step2l(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
     };
     // backward step into position t with the composition phi += Gb(t) Gf(t)
     auto bwd = [&](int t, const double *in, double *out, const double *gf) {
@@ -1307,8 +1328,7 @@ int sfgpu_system::molecule_phi(int m) {
             launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg],
                        pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], (int)COMP_ACC, 1, (int)STEP2_PLAIN);
         else
-            step2l_rows<<<grid_rows(L), kBlock, 0, s>>>(L, in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf,
-                                        o.d_phi[sg], COMP_ACC, 1);
+            launch_step2l(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
     };
     const bool ori = orient && K > 1;
     // storage: every slice, or checkpoints ck[q] = Gf(qk) plus one segment
@@ -1849,8 +1869,7 @@ extern "C" int sfgpu_lat_propagate(sfgpu_system *s, const double *gin, const dou
     else if (s->K == 6)
         step2<<<gr, kBlock, 0, s->stream>>>(s->H.L, gin, g, S, gout, nullptr, nullptr, COMP_NONE, backward);
     else
-        step2l_rows<<<grid_rows(s->H.L), kBlock, 0, s->stream>>>(s->H.L, gin, g, S, gout, nullptr, nullptr, COMP_NONE,
-                                                                backward);
+        return s->launch_step2l(gin, g, S, gout, nullptr, nullptr, COMP_NONE, backward);
     SFGPU_CUDA_TRY(cudaGetLastError());
     return SFGPU_OK;
 }

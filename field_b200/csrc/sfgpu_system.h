@@ -150,6 +150,8 @@ struct sfgpu_system {
     int chi_vjp_async(const double *x, const double *w, double *dchi);
     std::vector<double *> a_phibar_m;
     int vjp_async(const double *x, const double *w, double *f, double *xbar);
+    int launch_step2l(const double *gin, const double *G, double S, double *gout, const double *other, double *phi,
+                      int mode, int backward);
     int launch_step1(const double *gin, const double *G, double *gout, const double *other, double *phi, int mode);
     // overflow protection: chain statistics in logarithms (first-order 1D/2D)
     bool logmode = false;

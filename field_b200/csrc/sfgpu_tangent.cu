@@ -234,7 +234,7 @@ int sfgpu_system::molecule_phi_t(int m) {
                                                  iso ? STEP2_ISO : STEP2_STIFF);
             } else {
                 const double Sv = backward ? pf[sg * nseg + o.seg[t + 1]] : pf[o.seg[t - 1] * nseg + sg];
-                step2l_rows<<<gr, kBlock, 0, s>>>(L, in, G, Sv, out, nullptr, nullptr, COMP_NONE, backward ? 1 : 0);
+                launch_step2l(in, G, Sv, out, nullptr, nullptr, COMP_NONE, backward ? 1 : 0);
             }
         };
         auto pair_step = [&](int t, bool backward, const double *in, const double *din, double *out, double *dout) {
