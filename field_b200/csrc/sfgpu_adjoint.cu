@@ -540,15 +540,12 @@ int sfgpu_system::molecule_adjoint(int m, double *const *phibar_src) {
     auto GB = [&](int j) -> const double * { return (a_stride ? a_bufB : a_gb) + (size_t)j * KM; };
     if (K == 1 && o.force == 0 && !lat_twelve(L)) {
         // gathering sweeps (adj_gather_*): cot and nxt hold y
-        const int XC = 8;   // planes a block marches through: as the composing primal step's
         auto step = [&](int t, const double *y, const double *P, const double *Q, bool lngn) -> int {
             const int sg = o.seg[t];
             AdjStep a{y, a_phibar_raw[sg], P, d_gseg[sg], Q, lngn ? d_wgn : nullptr, a_qbar, a_h[sg], nxt};
             cudaError_t e;
             if (L.grad == 3) {
-                const dim3 grid((L.Md[2] - 2 + kTZ - 1) / kTZ, (L.Md[1] - 2 + kTY - 1) / kTY, (L.Md[0] - 2 + XC - 1) / XC);
-                e = y ? launch_pdl(adj_gather_march<false>, grid, dim3(kTZ * kTY), s, L, a, XC)
-                      : launch_pdl(adj_gather_march<true>, grid, dim3(kTZ * kTY), s, L, a, XC);
+                e = launch_pdl(y ? adj_gather_cols<false> : adj_gather_cols<true>, cols_grid(L), dim3(32, kColY), s, L, a);
             } else {
                 e = launch_pdl(adj_gather_rows, dim3(gr), dim3(kBlock), s, L, a);
             }

@@ -174,7 +174,7 @@ static __global__ void adj_chain_step(DLat L, const double *__restrict__ cot, co
 // Bound by memory: y, P', phibar_raw', G', Q', H' read, y', H' written, 64 B a
 // site and step.  The scatter it replaces took 6 FP64 atomics a site, a pass
 // of its own for phibar_raw . P and the stencil of the slice: 46 + 9 us a step
-// on a 128^3 lattice, 26 now.
+// on a 128^3 lattice, 22 now.
 
 // weight with which A^T at coordinate s of gradient d takes the lower / upper
 // neighbour (index lat_mapc of s -+ 1), for a step of weight 1 to either side
@@ -237,88 +237,48 @@ static __global__ void adj_gather_rows(DLat L, AdjStep a) {
     });
 }
 
-// the same on the six-neighbour 3D lattices, marching through x as
-// step3d_march_pf does (a 32 x 8 tile of columns, plane x + 1's loads in
-// flight while plane x is computed)
+// the same on the six-neighbour 3D lattices, in the columns of step3d_cols
 template <bool kStart>
-static __global__ void __launch_bounds__(kTZ * kTY, 3) adj_gather_march(DLat L, AdjStep o, int xc) {
-    __shared__ double tile[2][kTY + 2][kTZ + 2];
+static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols(DLat L, AdjStep o) {
     sfk::pdl_enter();
-    const int nx = L.Md[0] - 2, ny = L.Md[1] - 2, nz = L.Md[2] - 2;
-    const int jx = L.st[0], jy = L.st[1];
-    const int tz = threadIdx.x % kTZ, ty = threadIdx.x / kTZ;
-    const int z = blockIdx.x * kTZ + tz + 1;
-    const int y = blockIdx.y * kTY + ty + 1;
-    const int x0 = blockIdx.z * xc + 1;
-    if (x0 > nx) return;
-    const int x1 = min(x0 + xc - 1, nx);
-    const bool act = (z <= nz) && (y <= ny);
-    const int zm = lat_mapc(L, 2, z - 1), zp = lat_mapc(L, 2, z + 1);
-    const int ym = lat_mapc(L, 1, y - 1), yp = lat_mapc(L, 1, y + 1);
-    const bool hz0 = (tz == 0), hz1 = (tz == kTZ - 1) || (z == nz);
-    const bool hy0 = (ty == 0), hy1 = (ty == kTY - 1) || (y == ny);
-    const int col = y * jy + z;
-    const double wzl = act ? gather_lo(L, 2, z) * (1.0 / 6.0) : 0.0, wzh = act ? gather_hi(L, 2, z) * (1.0 / 6.0) : 0.0;
-    const double wyl = act ? gather_lo(L, 1, y) * (1.0 / 6.0) : 0.0, wyh = act ? gather_hi(L, 1, y) * (1.0 / 6.0) : 0.0;
-    double vprev = 0, vcur = 0, vnext = 0, hzl = 0, hzh = 0, hyl = 0, hyh = 0, g = 0, pr = 0, P = 0, Q = 0, H = 0;
-    auto load = [&](int x, double &g_, double &pr_, double &P_, double &Q_, double &H_) {
-        const int t = x * jx + col;
-        g_ = o.G[t]; pr_ = o.pr[t]; P_ = o.P[t]; Q_ = o.Q[t]; H_ = o.H[t];
-    };
-    auto halos = [&](int x, double &a, double &b, double &c, double &d) {
-        const int base = x * jx;
-        if (hz0) a = o.y[base + y * jy + zm];
-        if (hz1) b = o.y[base + y * jy + zp];
-        if (hy0) c = o.y[base + ym * jy + z];
-        if (hy1) d = o.y[base + yp * jy + z];
-    };
-    if (act) {
-        load(x0, g, pr, P, Q, H);
-        if (!kStart) {
-            vprev = o.y[lat_mapc(L, 0, x0 - 1) * jx + col];
-            vcur = o.y[x0 * jx + col];
-            vnext = o.y[lat_mapc(L, 0, x0 + 1) * jx + col];
-            halos(x0, hzl, hzh, hyl, hyh);
-        }
-    }
+    const Column c(L);
+    if (!c.in) return;
+    const int nx = L.Md[0] - 2;
+    const int z = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * kColY + threadIdx.y + 1;
+    const double s6 = 1.0 / 6.0;
+    const double wzl = gather_lo(L, 2, z) * s6, wzh = gather_hi(L, 2, z) * s6;
+    const double wyl = gather_lo(L, 1, y) * s6, wyh = gather_hi(L, 1, y) * s6;
     const double qb = (kStart && o.w) ? *o.qbar : 0.0;
-    int b = 0;
-    for (int x = x0; x <= x1; x++) {
-        double vn2 = 0, nzl = 0, nzh = 0, nyl = 0, nyh = 0, gn = 0, prn = 0, Pn = 0, Qn = 0, Hn = 0;
-        if (act && x < x1) {
-            load(x + 1, gn, prn, Pn, Qn, Hn);
-            if (!kStart) {
-                vn2 = o.y[lat_mapc(L, 0, x + 2) * jx + col];
-                halos(x + 1, nzl, nzh, nyl, nyh);
-            }
+    double v[kCols + 2];
+    if (!kStart) c.planes(L, o.y, v);
+#pragma unroll
+    for (int u0 = 0; u0 < kCols; u0 += 2) {      // two planes' other loads at a time
+        double a[2][4], g[2], pr[2], P[2], Q[2], H[2], w[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int x = c.x0 + u0 + e;
+            if (x > nx) continue;
+            const int t = x * L.st[0] + c.col;
+            if (!kStart) c.sides(o.y, t, a[e]);
+            pr[e] = o.pr[t]; P[e] = o.P[t]; Q[e] = o.Q[t]; g[e] = o.G[t]; H[e] = o.H[t];
+            w[e] = (kStart && o.w) ? o.w[t] : 0.0;
         }
-        if (!kStart) {
-            if (act) {
-                tile[b][ty + 1][tz + 1] = vcur;
-                if (hz0) tile[b][ty + 1][0] = hzl;
-                if (hz1) tile[b][ty + 1][tz + 2] = hzh;
-                if (hy0) tile[b][0][tz + 1] = hyl;
-                if (hy1) tile[b][ty + 2][tz + 1] = hyh;
-            }
-            __syncthreads();
-        }
-        if (act) {
-            const int t = x * jx + col;
-            double c = pr * P;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int u = u0 + e, x = c.x0 + u;
+            if (x > nx) continue;
+            const int t = x * L.st[0] + c.col;
+            double r = pr[e] * P[e];
             if (kStart) {
-                if (o.w) c += qb * o.w[t];
+                r += qb * w[e];
             } else {
-                c += (gather_lo(L, 0, x) * vprev + gather_hi(L, 0, x) * vnext) * (1.0 / 6.0);
-                c += wyl * tile[b][ty][tz + 1] + wyh * tile[b][ty + 2][tz + 1];
-                c += wzl * tile[b][ty + 1][tz] + wzh * tile[b][ty + 1][tz + 2];
+                r += (gather_lo(L, 0, x) * v[u] + gather_hi(L, 0, x) * v[u + 2]) * s6;
+                r += wyl * a[e][0] + wyh * a[e][1];
+                r += wzl * a[e][2] + wzh * a[e][3];
             }
-            o.H[t] = H + c * Q;
-            o.out[t] = g * c;
+            o.H[t] = H[e] + r * Q[e];
+            o.out[t] = g[e] * r;
         }
-        vprev = vcur; vcur = vnext; vnext = vn2;
-        hzl = nzl; hzh = nzh; hyl = nyl; hyh = nyh;
-        g = gn; pr = prn; P = Pn; Q = Qn; H = Hn;
-        b ^= 1;
     }
 }
 

@@ -388,6 +388,82 @@ step3d_march_pf2(DLat L, const double *__restrict__ gin, const double *__restric
     }
 }
 
+// The six-neighbour 3D step without a tile: a thread owns kCols consecutive x
+// planes of one (y, z) column, a block 32 (z) x kColY (y) columns.  The column's
+// kCols + 2 values come once from L2, the y and z neighbours are other threads'
+// own values and hit L1, and all of a thread's loads (about 7 a site, 34 for
+// four forward sites) are in flight together: no barrier and no march, whose
+// planes waited for one another's latency.  What bounds it now is L2: 7.3 TB/s
+// of algorithmic bytes in the composing step.  Measured on 128^3 (us, march ->
+// this): forward 13.8 -> 9.8, backward 17.8 -> 14.4; on 90 x 75 x 61: 6.1 -> 3.6,
+// 7.1 -> 4.2; on 64^3: 4.8 -> 3.4, 5.9 -> 3.5.  Two planes a thread lose 10 %, eight
+// 10-40 % (registers), blocks of eight rows 5 %.  Operands and order as
+// step3d_march: bit-identical.
+constexpr int kCols = 4, kColY = 4;
+struct Column {              // a thread's columns: site of plane x is x * jx + col
+    int x0, col, oy[2], oz[2];
+    bool in;
+    __device__ __forceinline__ Column(const DLat &L) {
+        const int ny = L.Md[1] - 2, nz = L.Md[2] - 2;
+        const int z = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * kColY + threadIdx.y + 1;
+        x0 = blockIdx.z * kCols + 1;
+        in = z <= nz && y <= ny;
+        col = y * L.st[1] + z;
+        oy[0] = (lat_mapc(L, 1, y - 1) - y) * L.st[1];
+        oy[1] = (lat_mapc(L, 1, y + 1) - y) * L.st[1];
+        oz[0] = lat_mapc(L, 2, z - 1) - z;
+        oz[1] = lat_mapc(L, 2, z + 1) - z;
+    }
+    // the column's values at planes x0 - 1 .. x0 + kCols
+    __device__ __forceinline__ void planes(const DLat &L, const double *__restrict__ p, double (&v)[kCols + 2]) const {
+#pragma unroll
+        for (int u = 0; u < kCols + 2; u++)
+            v[u] = (x0 - 1 + u < L.Md[0]) ? p[lat_mapc(L, 0, x0 - 1 + u) * L.st[0] + col] : 0.0;
+    }
+    __device__ __forceinline__ void sides(const double *__restrict__ p, int t, double (&a)[4]) const {
+        a[0] = p[t + oy[0]]; a[1] = p[t + oy[1]]; a[2] = p[t + oz[0]]; a[3] = p[t + oz[1]];
+    }
+};
+inline dim3 cols_grid(const DLat &L) {
+    return dim3((L.Md[2] - 2 + 31) / 32, (L.Md[1] - 2 + kColY - 1) / kColY, (L.Md[0] - 2 + kCols - 1) / kCols);
+}
+
+template <int kMode>
+static __global__ void __launch_bounds__(32 * kColY, 6)
+step3d_cols(DLat L, const double *__restrict__ gin, const double *__restrict__ G, double *__restrict__ gout,
+            const double *__restrict__ other, double *__restrict__ phi) {
+    pdl_enter();
+    const Column c(L);
+    if (!c.in) return;
+    const int nx = L.Md[0] - 2;
+    double v[kCols + 2], a[kCols][4], g[kCols], ot[kCols], ph[kCols];
+    c.planes(L, gin, v);
+#pragma unroll
+    for (int u = 0; u < kCols; u++) {
+        if (c.x0 + u > nx) continue;
+        const int t = (c.x0 + u) * L.st[0] + c.col;
+        g[u] = G[t];
+        c.sides(gin, t, a[u]);
+        if (kMode == COMP_ACC) ot[u] = other[t];
+        if (kMode != COMP_NONE) ph[u] = phi[t];
+    }
+#pragma unroll
+    for (int u = 0; u < kCols; u++) {
+        if (c.x0 + u > nx) continue;
+        const int t = (c.x0 + u) * L.st[0] + c.col;
+        double acc = v[u] * g[u];
+        acc += v[u + 2] * g[u];
+        acc += a[u][0] * g[u];
+        acc += a[u][1] * g[u];
+        acc += a[u][2] * g[u];
+        acc += a[u][3] * g[u];
+        const double out = acc * (1.0 / 6.0);
+        gout[t] = out;
+        if (kMode == COMP_ACC) phi[t] = ph[u] + out * ot[u];
+        else if (kMode == COMP_CENTRE) phi[t] = (ph[u] + out * out) * 0.5;
+    }
+}
+
 // One second-order step (Lat3D2ndO::PropagateF, Lat3D2ndO.cpp:65-152, and
 // PropagateB, :597-678) for the six direction components, with boundary
 // components swapped at mirrors (SetBx1(gz0,gz5)..., Lat3D2ndO.cpp:84-89) and

@@ -56,7 +56,11 @@ int sfgpu_system::launch_step1(const double *gin, const double *G, double *gout,
         dim3 grid((L.Md[2] - 2 + kTZ - 1) / kTZ, (L.Md[1] - 2 + kTY - 1) / kTY, (L.Md[0] - 2 + xc - 1) / xc);
         const dim3 block(kTZ * kTY);
         cudaError_t e;
-        if (!composing && tile_pipelined == 2) {
+        if ((composing ? tile_pipelined_bwd : tile_pipelined) == 3) {
+            auto k = mode == COMP_ACC ? step3d_cols<COMP_ACC>
+                                      : mode == COMP_CENTRE ? step3d_cols<COMP_CENTRE> : step3d_cols<COMP_NONE>;
+            e = launch_pdl(k, cols_grid(L), dim3(32, kColY), stream, L, gin, G, gout, other, phi);
+        } else if (!composing && tile_pipelined == 2) {
             grid.y = (L.Md[1] - 2 + kTY2 - 1) / kTY2;
             e = launch_pdl(step3d_march_pf2, grid, block, stream, L, gin, G, gout, xc);
         } else if (composing && tile_pipelined_bwd) {
@@ -2047,20 +2051,21 @@ extern "C" int sfgpu_system_autotune(sfgpu_system *s, int reps, int *chosen_xc, 
     // forward and backward steps are timed by the same profile call; each
     // keeps its own fastest (depth, form)
     // forms: 0 plain, 1 pipelined, 2 (forward only) pipelined with two y rows
-    // per thread
+    // per thread, 3 columns without a march
     const int cand[] = {2, 4, 8, 16, 32};
     double bf = 1e30, bb = 1e30;
     int fx = s->tile_xc, fp = s->tile_pipelined, bx = s->tile_xc_bwd, bp = s->tile_pipelined_bwd;
-    for (int pl = 0; pl < 3; pl++)
+    for (int pl = 0; pl < 4; pl++)
         for (int c : cand) {
             s->tile_xc = s->tile_xc_bwd = c;
             s->tile_pipelined = pl;
-            s->tile_pipelined_bwd = pl != 0;
+            s->tile_pipelined_bwd = pl == 2 ? 1 : pl;
             double f = 0, b = 0;
             int rc = sfgpu_profile_propagator(s, reps, &f, &b, nullptr, nullptr);
             if (rc) return rc;
             if (f < bf) { bf = f; fx = c; fp = pl; }
-            if (pl < 2 && b < bb) { bb = b; bx = c; bp = pl; }
+            if (pl != 2 && b < bb) { bb = b; bx = c; bp = pl; }
+            if (pl == 3) break;   // no depth to choose
         }
     s->tile_xc = fx; s->tile_pipelined = fp;
     s->tile_xc_bwd = bx; s->tile_pipelined_bwd = bp;
@@ -2081,5 +2086,8 @@ extern "C" int sfgpu_system_set_tile(sfgpu_system *s, int xc) {
     CHECK_SYS(s);
     if (xc < 1 || xc > 1024) return fail(SFGPU_ERR_INVALID, "tile depth must be in 1..1024");
     s->tile_xc = s->tile_xc_bwd = xc;
+    // a depth is a march's
+    if (s->tile_pipelined == 3) s->tile_pipelined = 0;
+    if (s->tile_pipelined_bwd == 3) s->tile_pipelined_bwd = 1;
     return SFGPU_OK;
 }

@@ -82,10 +82,11 @@ struct sfgpu_system {
     double *d_x = nullptr, *d_f = nullptr;
     int nblocks_red = 1;
     // 3D first-order step, separately for the composition-free forward steps
-    // and the composing backward steps: x planes per block and whether the
-    // software-pipelined form (step3d_march_pf) runs it
+    // and the composing backward steps: the form (3: step3d_cols; the marches:
+    // 0 plain, 1 pipelined, 2 pipelined with two rows, forward only) and the
+    // x planes a block of a march walks
     int tile_xc = 4, tile_xc_bwd = 8;
-    int tile_pipelined = 0, tile_pipelined_bwd = 1;
+    int tile_pipelined = 3, tile_pipelined_bwd = 3;
     // chain storage of residual evaluations: 0 keeps every forward slice,
     // k > 0 keeps every k-th one and recomputes the others segment by
     // segment during the backward sweep (set at creation)
@@ -150,6 +151,8 @@ struct sfgpu_system {
     int chi_vjp_async(const double *x, const double *w, double *dchi);
     std::vector<double *> a_phibar_m;
     int vjp_async(const double *x, const double *w, double *f, double *xbar);
+    int launch_step1_t(const double *gin, const double *dgin, const double *G, const double *dG, double *gout,
+                       double *dgout, const double *other, const double *dother, double *phi, double *dphi, int mode);
     int launch_step2l(const double *gin, const double *G, double S, double *gout, const double *other, double *phi,
                       int mode, int backward);
     int launch_step1(const double *gin, const double *G, double *gout, const double *other, double *phi, int mode);

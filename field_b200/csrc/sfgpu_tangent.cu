@@ -74,6 +74,24 @@ int sfgpu_system::ensure_tangent() {
     return SFGPU_OK;
 }
 
+// first-order step with its tangent, a programmatic dependent of the one before
+int sfgpu_system::launch_step1_t(const double *gin, const double *dgin, const double *G, const double *dG, double *gout,
+                                 double *dgout, const double *other, const double *dother, double *phi, double *dphi,
+                                 int mode) {
+    const DLat &L = H.L;
+    cudaError_t e;
+    if (L.grad == 3 && !lat_twelve(L)) {
+        auto k = mode == COMP_ACC ? step3d_cols_t<COMP_ACC>
+                                  : mode == COMP_CENTRE ? step3d_cols_t<COMP_CENTRE> : step3d_cols_t<COMP_NONE>;
+        e = launch_pdl(k, cols_grid(L), dim3(32, kColY), stream, L, gin, dgin, G, dG, gout, dgout, other, dother, phi, dphi);
+    } else {
+        e = launch_pdl(step1_rows_t, dim3(grid_rows_t(L)), dim3(kBlock), stream, L, gin, dgin, G, dG, gout, dgout, other,
+                       dother, phi, dphi, mode);
+    }
+    if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+    return SFGPU_OK;
+}
+
 int sfgpu_system::molecule_phi_t(int m) {
     if (mols[m].dend) {
         // a dendrimer's derivatives: the bond-tree recursion on its tree form
@@ -139,8 +157,8 @@ int sfgpu_system::molecule_phi_t(int m) {
             SFGPU_CUDA_TRY(cudaMemsetAsync(o.d_dphi[i], 0, bytes, s));
         }
         auto stepT = [&](const double *in, const double *din, int sgq, double *out, double *dout) {
-            step1_rows_t<<<gr, kBlock, 0, s>>>(L, in, din, d_gseg[sgq], dgseg[sgq], out, dout, nullptr, nullptr,
-                                               nullptr, nullptr, COMP_NONE);
+            launch_step1_t(in, din, d_gseg[sgq], dgseg[sgq], out, dout, nullptr, nullptr,
+                           nullptr, nullptr, COMP_NONE);
         };
         for (int q = N - 1; q >= 0; q--) {
             const int sq = o.seg[q];
@@ -200,20 +218,20 @@ int sfgpu_system::molecule_phi_t(int m) {
         SFGPU_CUDA_TRY(cudaMemcpyAsync(t_gi, G, sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         SFGPU_CUDA_TRY(cudaMemcpyAsync(d_dgi, dG, sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         for (int t = 1; t < half; t++)
-            step1_rows_t<<<gr, kBlock, 0, s>>>(L, t_gi + (size_t)(t - 1) * M, d_dgi + (size_t)(t - 1) * M, G, dG,
-                                               t_gi + (size_t)t * M, d_dgi + (size_t)t * M, nullptr, nullptr,
-                                               nullptr, nullptr, COMP_NONE);
+            launch_step1_t(t_gi + (size_t)(t - 1) * M, d_dgi + (size_t)(t - 1) * M, G, dG,
+                           t_gi + (size_t)t * M, d_dgi + (size_t)t * M, nullptr, nullptr,
+                           nullptr, nullptr, COMP_NONE);
         cur = t_gi + (size_t)(half - 1) * M;
         dcur = d_dgi + (size_t)(half - 1) * M;
         if (N % 2 == 1) {
-            step1_rows_t<<<gr, kBlock, 0, s>>>(L, cur, dcur, G, dG, ginv, dginv, nullptr, nullptr, phi, dph, COMP_CENTRE);
+            launch_step1_t(cur, dcur, G, dG, ginv, dginv, nullptr, nullptr, phi, dph, COMP_CENTRE);
             cur = ginv; dcur = dginv;
             std::swap(ginv, tmp); std::swap(dginv, dtmp);
         }
         for (int sp = (N + 3) / 2; sp <= N; sp++) {
             int sinv = N - sp + 1;
-            step1_rows_t<<<gr, kBlock, 0, s>>>(L, cur, dcur, G, dG, ginv, dginv, t_gi + (size_t)(sinv - 1) * M,
-                                               d_dgi + (size_t)(sinv - 1) * M, phi, dph, COMP_ACC);
+            launch_step1_t(cur, dcur, G, dG, ginv, dginv, t_gi + (size_t)(sinv - 1) * M,
+                           d_dgi + (size_t)(sinv - 1) * M, phi, dph, COMP_ACC);
             cur = ginv; dcur = dginv;
             std::swap(ginv, tmp); std::swap(dginv, dtmp);
         }
@@ -256,8 +274,8 @@ int sfgpu_system::molecule_phi_t(int m) {
                 step1_force_rows_t<<<gr, kBlock, 0, s>>>(L, force_weights(L, o.force), src, dsrc, d_gseg[sg], dgseg[sg],
                                                          dst, ddst, nullptr, nullptr, nullptr, nullptr, COMP_NONE);
             else if (K == 1)
-                step1_rows_t<<<gr, kBlock, 0, s>>>(L, src, dsrc, d_gseg[sg], dgseg[sg], dst, ddst, nullptr, nullptr,
-                                                   nullptr, nullptr, COMP_NONE);
+                launch_step1_t(src, dsrc, d_gseg[sg], dgseg[sg], dst, ddst, nullptr, nullptr,
+                           nullptr, nullptr, COMP_NONE);
             else
                 step2_rows_t<<<gr, kBlock, 0, s>>>(L, src, dsrc, d_gseg[sg], dgseg[sg], pf[o.seg[t - 1] * nseg + sg],
                                                    dst, ddst, nullptr, nullptr, nullptr, nullptr, COMP_NONE, 0);
@@ -279,9 +297,9 @@ int sfgpu_system::molecule_phi_t(int m) {
                                                          dgseg[sg], ginv, dginv, t_gi + (size_t)t * KM,
                                                          d_dgi + (size_t)t * KM, o.d_phi[sg], o.d_dphi[sg], COMP_ACC);
             else if (K == 1)
-                step1_rows_t<<<gr, kBlock, 0, s>>>(L, cur, dcur, d_gseg[sg], dgseg[sg], ginv, dginv,
-                                                   t_gi + (size_t)t * KM, d_dgi + (size_t)t * KM, o.d_phi[sg],
-                                                   o.d_dphi[sg], COMP_ACC);
+                launch_step1_t(cur, dcur, d_gseg[sg], dgseg[sg], ginv, dginv,
+                           t_gi + (size_t)t * KM, d_dgi + (size_t)t * KM, o.d_phi[sg],
+                           o.d_dphi[sg], COMP_ACC);
             else
                 step2_rows_t<<<gr, kBlock, 0, s>>>(L, cur, dcur, d_gseg[sg], dgseg[sg], pf[sg * nseg + o.seg[t + 1]],
                                                    ginv, dginv, t_gi + (size_t)t * KM, d_dgi + (size_t)t * KM,

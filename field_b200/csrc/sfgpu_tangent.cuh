@@ -75,6 +75,7 @@ static __global__ void step1_rows_t(DLat L, const double *__restrict__ gin, cons
                                     double *__restrict__ gout, double *__restrict__ dgout,
                                     const double *__restrict__ other, const double *__restrict__ dother,
                                     double *__restrict__ phi, double *__restrict__ dphi, int mode) {
+    pdl_enter();
     const int worker = blockIdx.x * blockDim.x + threadIdx.x;
     for_interior(L, worker, gridDim.x * blockDim.x, [&](const RowInfo &R, int k, int nlast) {
         const int t = R.base + k;
@@ -90,6 +91,65 @@ static __global__ void step1_rows_t(DLat L, const double *__restrict__ gin, cons
             dphi[t] = (dphi[t] + 2.0 * out * dout) * 0.5;
         }
     });
+}
+
+// step1_rows_t on the six-neighbour 3D lattices, in the columns of
+// step3d_cols: 90 x 75 x 61, 13.5 us a step by rows, 5.9 this way.
+// Same operands and order, bit-identical.
+template <int kMode>
+static __global__ void __launch_bounds__(32 * kColY, 4)
+step3d_cols_t(DLat L, const double *__restrict__ gin, const double *__restrict__ dgin, const double *__restrict__ G,
+              const double *__restrict__ dG, double *__restrict__ gout, double *__restrict__ dgout,
+              const double *__restrict__ other, const double *__restrict__ dother, double *__restrict__ phi,
+              double *__restrict__ dphi) {
+    pdl_enter();
+    const Column c(L);
+    if (!c.in) return;
+    const int nx = L.Md[0] - 2;
+    double v[kCols + 2], w[kCols + 2];
+    c.planes(L, gin, v);
+    c.planes(L, dgin, w);
+#pragma unroll
+    for (int u0 = 0; u0 < kCols; u0 += 2) {      // two planes' side loads at a time
+        double a[2][4], b[2][4], g[2], dg[2], ot[2], dot[2], ph[2], dp[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int u = u0 + e;
+            if (c.x0 + u > nx) continue;
+            const int t = (c.x0 + u) * L.st[0] + c.col;
+            g[e] = G[t];
+            dg[e] = dG[t];
+            c.sides(gin, t, a[e]);
+            c.sides(dgin, t, b[e]);
+            if (kMode == COMP_ACC) { ot[e] = other[t]; dot[e] = dother[t]; }
+            if (kMode != COMP_NONE) { ph[e] = phi[t]; dp[e] = dphi[t]; }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int u = u0 + e;
+            if (c.x0 + u > nx) continue;
+            const int t = (c.x0 + u) * L.st[0] + c.col;
+            double acc = v[u] * g[e];
+            acc += v[u + 2] * g[e];
+            acc += a[e][0] * g[e];
+            acc += a[e][1] * g[e];
+            acc += a[e][2] * g[e];
+            acc += a[e][3] * g[e];
+            const double out = acc * (1.0 / 6.0);
+            const double raw = (v[u] + v[u + 2] + a[e][0] + a[e][1] + a[e][2] + a[e][3]) * (1.0 / 6.0);
+            const double draw = (w[u] + w[u + 2] + b[e][0] + b[e][1] + b[e][2] + b[e][3]) * (1.0 / 6.0);
+            const double dout = dg[e] * raw + g[e] * draw;
+            gout[t] = out;
+            dgout[t] = dout;
+            if (kMode == COMP_ACC) {
+                phi[t] = ph[e] + out * ot[e];
+                dphi[t] = dp[e] + (dout * ot[e] + out * dot[e]);
+            } else if (kMode == COMP_CENTRE) {
+                phi[t] = (ph[e] + out * out) * 0.5;
+                dphi[t] = (dp[e] + 2.0 * out * dout) * 0.5;
+            }
+        }
+    }
 }
 
 // primal constant-force step (as step1_force_rows) plus its tangent: the
