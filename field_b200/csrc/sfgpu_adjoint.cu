@@ -135,7 +135,7 @@ struct SwfAdj {
     int cls[SFGPU_MAX_SEG];
     int pinned[SFGPU_MAX_SEG];
     const double *gbar[SFGPU_MAX_SEG], *gfull[SFGPU_MAX_SEG], *range[SFGPU_MAX_SEG];
-    const double *h[SFGPU_MAX_SEG];   // Gbar . G collected as a product (adj_gather_*)
+    const double *h[SFGPU_MAX_SEG], *h2[SFGPU_MAX_SEG];   // Gbar . G collected as products, a sweep each (adj_gather_*)
 };
 __global__ void adj_swf(int nsites, SwfAdj sa, const int *__restrict__ sites, double *__restrict__ xbar) {
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nsites; j += gridDim.x * blockDim.x) {
@@ -144,7 +144,7 @@ __global__ void adj_swf(int nsites, SwfAdj sa, const int *__restrict__ sites, do
             if (sa.cls[i] < 0) continue;
             double gb = sa.gbar[i][z];
             if (sa.pinned[i] && !(sa.range[i][z] > 0)) gb = 0;
-            xbar[(size_t)j * sa.nclass + sa.cls[i]] -= gb * sa.gfull[i][z] + sa.h[i][z];
+            xbar[(size_t)j * sa.nclass + sa.cls[i]] -= gb * sa.gfull[i][z] + (sa.h[i][z] + sa.h2[i][z]);
         }
     }
 }
@@ -156,12 +156,19 @@ int sfgpu_system::ensure_adjoint_misc() {
     int rc;
     if (!a_misc) {
         a_phibar.assign(nseg, nullptr); a_gbar.assign(nseg, nullptr); a_phibar_raw.assign(nseg, nullptr); a_h.assign(nseg, nullptr);
+        a_h2.assign(nseg, nullptr);
         for (int i = 0; i < nseg; i++) {
             if ((rc = alloc_d(&a_phibar[i], M)) || (rc = alloc_d(&a_gbar[i], M)) ||
-                (rc = alloc_d(&a_phibar_raw[i], M)) || (rc = alloc_d(&a_h[i], M)))
+                (rc = alloc_d(&a_phibar_raw[i], M)) || (rc = alloc_d(&a_h[i], M)) ||
+                (rc = alloc_d(&a_h2[i], M)))
                 return rc;
         }
         if ((rc = alloc_d(&a_cot[0], (size_t)K * M)) || (rc = alloc_d(&a_cot[1], (size_t)K * M))) return rc;
+        if (K == 1 && ((rc = alloc_d(&a_cot2[0], M)) || (rc = alloc_d(&a_cot2[1], M)))) return rc;
+        if (K == 1) {
+            SFGPU_CUDA_TRY(cudaMemset(a_cot2[0], 0, sizeof(double) * M));
+            SFGPU_CUDA_TRY(cudaMemset(a_cot2[1], 0, sizeof(double) * M));
+        }
         // the gathering steps read surface layers, which no step writes
         SFGPU_CUDA_TRY(cudaMemset(a_cot[0], 0, sizeof(double) * K * M));
         SFGPU_CUDA_TRY(cudaMemset(a_cot[1], 0, sizeof(double) * K * M));
@@ -342,6 +349,12 @@ void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *ds
         launch_step2l(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
 }
 
+// Whether a stored chain's two sweeps run side by side: while what a reverse
+// step of each moves (64 B a site) stays in the 126 MB L2.  J^T w of a melt of
+// N = 30, one after the other / side by side: 24^3 468 / 287 us, 64^3 721 / 609,
+// 90^3 1297 / 1251, 100^3 1683 / 1770, 110^3 2039 / 2207.
+bool sfgpu_system::pair_sweeps() const { return 2 * 64.0 * M <= 100e6; }
+
 // Gf and Gb of every position of molecule m's chain (full chains, also for
 // symmetric homopolymers) into a_gf / a_gb; with compose, the backward sweep
 // also accumulates Gf.Gb into the molecule's (zeroed) phi.  *gb0 = Gb(0).
@@ -352,6 +365,42 @@ int sfgpu_system::store_chains(int m, bool compose, const double **gb0) {
     cudaStream_t s = stream;
     const int N = o.N;
     const size_t KM = (size_t)K * M;
+    if (K == 1 && o.force == 0 && !lat_twelve(H.L) && pair_sweeps()) {
+        // both recursions side by side, then the composition over the stored
+        // slices: half the launches, and phi is read and written once a run
+        // instead of once a step
+        adj_start(d_gseg[o.seg[0]], a_gf);
+        adj_start(d_gseg[o.seg[N - 1]], a_gb + (size_t)(N - 1) * M);
+        for (int i = 1; i < N; i++) {
+            const int b = N - 1 - i;
+            PairStep p{{a_gf + (size_t)(i - 1) * M, a_gb + (size_t)(b + 1) * M},
+                       {d_gseg[o.seg[i]], d_gseg[o.seg[b]]},
+                       {a_gf + (size_t)i * M, a_gb + (size_t)b * M}};
+            cudaError_t e;
+            if (H.L.grad == 3) {
+                dim3 grid = cols_grid(H.L);
+                const int nz = grid.z;
+                grid.z *= 2;
+                e = launch_pdl(step3d_cols_pair, grid, dim3(32, kColY), s, H.L, p, nz);
+            } else {
+                dim3 grid = sites_grid(H.L);
+                grid.z = 2;
+                e = launch_pdl(step1_sites_pair, grid, sites_block(H.L), s, H.L, p);
+            }
+            if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+        }
+        if (compose)
+            for (int hi = N - 1; hi >= 0;) {
+                int lo = hi;
+                while (lo > 0 && o.seg[lo - 1] == o.seg[hi]) lo--;
+                const cudaError_t e = launch_pdl(compose_run, dim3(g), dim3(kBlock), s, M, (const double *)a_gf,
+                                                 (const double *)a_gb, hi, lo, o.d_phi[o.seg[hi]]);
+                if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+                hi = lo - 1;
+            }
+        if (gb0) *gb0 = a_gb;
+        return SFGPU_OK;
+    }
     adj_start(d_gseg[o.seg[0]], a_gf);
     for (int t = 1; t < N; t++) adj_fstep(o, t, a_gf + (size_t)(t - 1) * KM, a_gf + (size_t)t * KM);
     adj_start(d_gseg[o.seg[N - 1]], a_gb + (size_t)(N - 1) * KM);
@@ -539,29 +588,59 @@ int sfgpu_system::molecule_adjoint(int m, double *const *phibar_src) {
     auto GF = [&](int j) -> const double * { return (a_stride ? a_bufF : a_gf) + (size_t)j * KM; };
     auto GB = [&](int j) -> const double * { return (a_stride ? a_bufB : a_gb) + (size_t)j * KM; };
     if (K == 1 && o.force == 0 && !lat_twelve(L)) {
-        // gathering sweeps (adj_gather_*): cot and nxt hold y
-        auto step = [&](int t, const double *y, const double *P, const double *Q, bool lngn) -> int {
+        // gathering sweeps (adj_gather_*).  With every slice stored the two run
+        // side by side, a launch taking a step of each; with checkpoints one
+        // after the other, as the segments' slices pass by.
+        auto make = [&](int q, int t, const double *y, double *out, const double *P, const double *Q, bool lngn) {
             const int sg = o.seg[t];
-            AdjStep a{y, a_phibar_raw[sg], P, d_gseg[sg], Q, lngn ? d_wgn : nullptr, a_qbar, a_h[sg], nxt};
+            return AdjStep{y, a_phibar_raw[sg], P, d_gseg[sg], Q, lngn ? d_wgn : nullptr, a_qbar,
+                           q ? a_h2[sg] : a_h[sg], out};
+        };
+        auto launch = [&](const AdjPair &p, int n) -> int {
             cudaError_t e;
+            const bool start = p.s[0].y == nullptr;
             if (L.grad == 3) {
-                e = launch_pdl(y ? adj_gather_cols<false> : adj_gather_cols<true>, cols_grid(L), dim3(32, kColY), s, L, a);
+                dim3 grid = cols_grid(L);
+                const int nzb = grid.z;
+                if (n == 2) {
+                    grid.z *= 2;
+                    e = launch_pdl(start ? adj_gather_cols_pair<true> : adj_gather_cols_pair<false>, grid,
+                                   dim3(32, kColY), s, L, p, nzb);
+                } else {
+                    e = launch_pdl(start ? adj_gather_cols<true> : adj_gather_cols<false>, grid, dim3(32, kColY), s, L,
+                                   p.s[0]);
+                }
             } else {
-                e = launch_pdl(adj_gather_rows, dim3(gr), dim3(kBlock), s, L, a);
+                dim3 grid = sites_grid(L);
+                grid.z = n;
+                e = launch_pdl(adj_gather_sites, grid, sites_block(L), s, L, p);
             }
-            std::swap(cot, nxt);
             if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
             return rcs;
         };
-        int rc = SFGPU_OK;
-        for (int t = N - 1; t >= 0 && !rc; t--) {      // forward recursion, descending
-            const int j = at(t);
-            rc = step(t, t == N - 1 ? nullptr : cot, GB(j), GF(j), false);
-        }
         adj_qbar_scale<<<1, 1, 0, s>>>(as, m, a_qbar);
-        for (int t = 0; t < N && !rc; t++) {           // backward recursion, ascending
-            const int j = at(t);
-            rc = step(t, t == 0 ? nullptr : cot, GF(j), GB(j), t == 0);
+        int rc = SFGPU_OK;
+        double *c2[2] = {a_cot2[0], a_cot2[1]};
+        if (a_stride == 0 && pair_sweeps()) {
+            for (int i = 0; i < N && !rc; i++) {
+                const int t = N - 1 - i, w = i & 1;
+                AdjPair p;
+                p.s[0] = make(0, t, i ? (w ? cot : nxt) : nullptr, w ? nxt : cot, GB(t), GF(t), false);
+                p.s[1] = make(1, i, i ? c2[w ^ 1] : nullptr, c2[w], GF(i), GB(i), i == 0);
+                rc = launch(p, 2);
+            }
+            return rc;
+        }
+        AdjPair p;
+        for (int i = 0; i < N && !rc; i++) {           // forward recursion, descending
+            const int t = N - 1 - i, j = at(t), w = i & 1;
+            p.s[0] = make(0, t, i ? (w ? cot : nxt) : nullptr, w ? nxt : cot, GB(j), GF(j), false);
+            rc = launch(p, 1);
+        }
+        for (int i = 0; i < N && !rc; i++) {           // backward recursion, ascending
+            const int j = at(i), w = i & 1;
+            p.s[0] = make(0, i, i ? (w ? cot : nxt) : nullptr, w ? nxt : cot, GF(j), GB(j), i == 0);
+            rc = launch(p, 1);
         }
         return rc;
     }
@@ -779,6 +858,7 @@ int sfgpu_system::vjp_async(const double *x, const double *w, double *f, double 
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_phibar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_gbar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_h[i], 0, sizeof(double) * M, s));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_h2[i], 0, sizeof(double) * M, s));
     }
     SFGPU_CUDA_TRY(cudaMemsetAsync(a_chibbar, 0, sizeof(double) * SFGPU_MAX_SEG, s));
     SFGPU_CUDA_TRY(cudaMemsetAsync(xbar, 0, sizeof(double) * nvar, s));
@@ -812,6 +892,7 @@ int sfgpu_system::vjp_async(const double *x, const double *w, double *f, double 
         sa.pinned[i] = freedom[i] == SFGPU_SEG_PINNED;
         sa.gbar[i] = a_gbar[i];
         sa.h[i] = a_h[i];
+        sa.h2[i] = a_h2[i];
         sa.gfull[i] = d_gfull[i];
         sa.range[i] = d_range[i];
     }
@@ -840,6 +921,7 @@ int sfgpu_system::free_energy_grad(const double *x, double *F, double *xbar) {
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_phibar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_gbar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_h[i], 0, sizeof(double) * M, s));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_h2[i], 0, sizeof(double) * M, s));
     }
     FeAdjParam fp;
     memset(&fp, 0, sizeof(fp));
@@ -885,6 +967,7 @@ int sfgpu_system::free_energy_grad(const double *x, double *F, double *xbar) {
         sa.pinned[i] = freedom[i] == SFGPU_SEG_PINNED;
         sa.gbar[i] = a_gbar[i];
         sa.h[i] = a_h[i];
+        sa.h2[i] = a_h2[i];
         sa.gfull[i] = d_gfull[i];
         sa.range[i] = d_range[i];
     }
@@ -904,6 +987,7 @@ int sfgpu_system::phi_vjp_async(const double *x, const double *const *omega, dou
         SFGPU_CUDA_TRY(cudaMemcpyAsync(a_phibar[i], omega[i], sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_gbar[i], 0, sizeof(double) * M, s));
         SFGPU_CUDA_TRY(cudaMemsetAsync(a_h[i], 0, sizeof(double) * M, s));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_h2[i], 0, sizeof(double) * M, s));
     }
     fe_zero_scal<<<1, 1, 0, s>>>(nmol, (AdjScal *)a_scal);
     int held = (mols[solvent].type != 0 && !mols[solvent].ring && !mols[solvent].tree && !mols[solvent].dend) ? solvent : -1;
@@ -928,6 +1012,7 @@ int sfgpu_system::phi_vjp_async(const double *x, const double *const *omega, dou
         sa.pinned[i] = freedom[i] == SFGPU_SEG_PINNED;
         sa.gbar[i] = a_gbar[i];
         sa.h[i] = a_h[i];
+        sa.h2[i] = a_h2[i];
         sa.gfull[i] = d_gfull[i];
         sa.range[i] = d_range[i];
     }

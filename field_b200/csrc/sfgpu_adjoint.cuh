@@ -224,25 +224,26 @@ struct AdjStep {
     const double *y, *pr, *P, *G, *Q, *w, *qbar;
     double *H, *out;
 };
-static __global__ void adj_gather_rows(DLat L, AdjStep a) {
+// two steps in one launch (the two sweeps of a chain whose slices are all
+// stored): grid.z, 2D and 1D; the second half of grid.z in 3D
+struct AdjPair { AdjStep s[2]; };
+static __global__ void __launch_bounds__(128) adj_gather_sites(DLat L, AdjPair p) {
     sfk::pdl_enter();
-    const int worker = blockIdx.x * blockDim.x + threadIdx.x;
-    for_interior(L, worker, gridDim.x * blockDim.x, [&](const RowInfo &R, int k, int nlast) {
+    const AdjStep &a = p.s[blockIdx.z];
+    for_site(L, [&](const RowInfo &R, int k, int nlast) {
         const int t = R.base + k;
-        double c = a.pr[t] * a.P[t];
+        const double P = a.P[t], pr = a.pr[t], Q = a.Q[t], H = a.H[t], g = a.G[t];
+        double c = pr * P;
         if (a.w) c += *a.qbar * a.w[t];
         if (a.y) c += gather1_row(L, R, a.y, k, nlast);
-        a.H[t] += c * a.Q[t];
-        a.out[t] = a.G[t] * c;
+        a.H[t] = H + c * Q;
+        a.out[t] = g * c;
     });
 }
 
 // the same on the six-neighbour 3D lattices, in the columns of step3d_cols
 template <bool kStart>
-static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols(DLat L, AdjStep o) {
-    sfk::pdl_enter();
-    const Column c(L);
-    if (!c.in) return;
+__device__ __forceinline__ void adj_cols(const DLat &L, const AdjStep &o, const Column &c) {
     const int nx = L.Md[0] - 2;
     const int z = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * kColY + threadIdx.y + 1;
     const double s6 = 1.0 / 6.0;
@@ -280,6 +281,21 @@ static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols(DLat L, 
             o.out[t] = g[e] * r;
         }
     }
+}
+template <bool kStart>
+static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols(DLat L, AdjStep o) {
+    sfk::pdl_enter();
+    const Column c(L);
+    if (c.in) adj_cols<kStart>(L, o, c);
+}
+template <bool kStart>
+static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols_pair(DLat L, AdjPair p, int nzb) {
+    sfk::pdl_enter();
+    const int q = blockIdx.z >= nzb;
+    Column c(L);
+    if (!c.in) return;
+    c.x0 -= q * nzb * kCols;
+    adj_cols<kStart>(L, p.s[q], c);
 }
 
 // out[k][t] = phibar_raw[t] * q[k][t] on interior sites (0 elsewhere), K components

@@ -277,6 +277,24 @@ __device__ __forceinline__ double prop1_row(const DLat &L, const RowInfo &R, con
     return acc * (1.0 / 6.0);
 }
 
+// The site-parallel walk of 1D and 2D lattices: one thread per interior site,
+// blocks of 32 x 4 sites (1D: 128), a warp along the last gradient.  Such a
+// lattice is a few thousand sites, and a step a latency: a row per warp leaves
+// most of the chip idle and its lanes walking (128 x 128 cylinder: reverse step
+// 11.7 us by rows, 4.4 by sites; forward step 5.8, 3.9).
+template <class F>
+__device__ __forceinline__ void for_site(const DLat &L, F &&f) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1, nlast = L.Md[L.grad - 1] - 2;
+    const int row = blockIdx.y * blockDim.y + threadIdx.y;
+    if (k > nlast || row >= lat_nrows(L)) return;
+    f(lat_row(L, row), k, nlast);
+}
+inline dim3 sites_block(const DLat &L) { return L.grad == 1 ? dim3(128) : dim3(32, 4); }
+inline dim3 sites_grid(const DLat &L) {
+    const int n = L.Md[L.grad - 1] - 2, rows = lat_nrows(L);
+    return L.grad == 1 ? dim3((n + 127) / 128) : dim3((n + 31) / 32, (rows + 3) / 4);
+}
+
 // Visit the interior sites assigned to this thread: for 1 gradient threads
 // stride over the single row; otherwise warps take rows and lanes take the
 // positions along the row.  worker = thread index among nworkers threads.

@@ -125,6 +125,23 @@ static __global__ void step1_rows(DLat L, const double *__restrict__ gin, const 
         });
 }
 
+// The same on 1D and 2D lattices, one thread per site, the composition's
+// operands loaded with the stencil's.
+template <int kMode>
+static __global__ void __launch_bounds__(128)
+step1_sites(DLat L, const double *__restrict__ gin, const double *__restrict__ G, double *__restrict__ gout,
+            const double *__restrict__ other, double *__restrict__ phi) {
+    pdl_enter();
+    for_site(L, [&](const RowInfo &R, int k, int nlast) {
+        const int t = R.base + k;
+        const double ot = (kMode == COMP_ACC) ? other[t] : 0.0, ph = (kMode != COMP_NONE) ? phi[t] : 0.0;
+        const double out = prop1_row<false>(L, R, gin, G, k, nlast);
+        gout[t] = out;
+        if (kMode == COMP_ACC) phi[t] = ph + out * ot;
+        else if (kMode == COMP_CENTRE) phi[t] = (ph + out * out) * 0.5;
+    });
+}
+
 // First-order step on a 3D lattice, x-marching: a block owns a 32 (z) x 8
 // (y) tile of columns and walks `xc` consecutive x planes.  The x-1/x/x+1
 // values of a column stay in registers, the y/z neighbours come from the
@@ -461,6 +478,70 @@ step3d_cols(DLat L, const double *__restrict__ gin, const double *__restrict__ G
         gout[t] = out;
         if (kMode == COMP_ACC) phi[t] = ph[u] + out * ot[u];
         else if (kMode == COMP_CENTRE) phi[t] = (ph[u] + out * out) * 0.5;
+    }
+}
+
+// Two independent composition-free steps in one launch, the blocks of the
+// second following those of the first in grid.z: the forward and the backward
+// recursion of a chain whose slices are all stored (half the launches of a
+// small lattice, whose steps are latency).  Operands and order as step1_sites
+// and step3d_cols.
+struct PairStep { const double *in[2], *G[2]; double *out[2]; };
+static __global__ void __launch_bounds__(128) step1_sites_pair(DLat L, PairStep p) {
+    pdl_enter();
+    const int q = blockIdx.z;
+    const double *gin = p.in[q], *G = p.G[q];
+    double *gout = p.out[q];
+    for_site(L, [&](const RowInfo &R, int k, int nlast) { gout[R.base + k] = prop1_row<false>(L, R, gin, G, k, nlast); });
+}
+static __global__ void __launch_bounds__(32 * kColY, 6) step3d_cols_pair(DLat L, PairStep p, int nz) {
+    pdl_enter();
+    const int q = blockIdx.z >= nz;
+    Column c(L);
+    if (!c.in) return;
+    c.x0 -= q * nz * kCols;
+    const int nx = L.Md[0] - 2;
+    const double *gin = p.in[q], *G = p.G[q];
+    double *gout = p.out[q];
+    double v[kCols + 2], a[kCols][4], g[kCols];
+    c.planes(L, gin, v);
+#pragma unroll
+    for (int u = 0; u < kCols; u++) {
+        if (c.x0 + u > nx) continue;
+        const int t = (c.x0 + u) * L.st[0] + c.col;
+        g[u] = G[t];
+        c.sides(gin, t, a[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kCols; u++) {
+        if (c.x0 + u > nx) continue;
+        double acc = v[u] * g[u];
+        acc += v[u + 2] * g[u];
+        acc += a[u][0] * g[u];
+        acc += a[u][1] * g[u];
+        acc += a[u][2] * g[u];
+        acc += a[u][3] * g[u];
+        gout[(c.x0 + u) * L.st[0] + c.col] = acc * (1.0 / 6.0);
+    }
+}
+
+// phi += Gb(t) Gf(t) for t = hi, hi - 1, ..., lo (one run of equal segments) of
+// stored slices, in the order in which composing steps add them
+static __global__ void compose_run(int M, const double *__restrict__ gf, const double *__restrict__ gb, int hi, int lo,
+                                   double *__restrict__ phi) {
+    pdl_enter();
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
+        double p = phi[r];
+        int t = hi;
+        for (; t - 7 >= lo; t -= 8) {
+            double a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) { a[u] = gb[(size_t)(t - u) * M + r]; b[u] = gf[(size_t)(t - u) * M + r]; }
+#pragma unroll
+            for (int u = 0; u < 8; u++) p = p + a[u] * b[u];
+        }
+        for (; t >= lo; t--) p = p + gb[(size_t)t * M + r] * gf[(size_t)t * M + r];
+        phi[r] = p;
     }
 }
 

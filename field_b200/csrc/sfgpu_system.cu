@@ -71,6 +71,11 @@ int sfgpu_system::launch_step1(const double *gin, const double *G, double *gout,
             e = launch_pdl(step3d_march, grid, block, stream, L, gin, G, gout, other, phi, mode, xc);
         }
         if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+    } else if (L.grad < 3) {
+        auto k = mode == COMP_ACC ? step1_sites<COMP_ACC>
+                                  : mode == COMP_CENTRE ? step1_sites<COMP_CENTRE> : step1_sites<COMP_NONE>;
+        const cudaError_t e = launch_pdl(k, sites_grid(L), sites_block(L), stream, L, gin, G, gout, other, phi);
+        if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
     } else {
         const cudaError_t e = launch_pdl(step1_rows, dim3(grid_rows(L)), dim3(kBlock), stream, L, gin, G, gout, other, phi,
                                          mode);

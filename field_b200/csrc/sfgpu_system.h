@@ -113,6 +113,7 @@ struct sfgpu_system {
     // reverse-mode (adjoint) buffers, allocated on the first J^T w
     bool a_ready = false;
     double *a_gf = nullptr, *a_gb = nullptr, *a_cot[2] = {nullptr, nullptr};
+    double *a_cot2[2] = {nullptr, nullptr};   // the ascending gathering sweep's
     // chain storage of the reverse sweep: every slice (a_stride 0) or
     // checkpoints every a_stride positions plus two segment buffers
     int a_stride = 0;
@@ -132,8 +133,9 @@ struct sfgpu_system {
     void dend_view(HMol &o, bool on);
     double *a_ckF = nullptr, *a_ckB = nullptr, *a_bufF = nullptr, *a_bufB = nullptr;
     int a_qseg = -1;                        // segment held in a_bufF / a_bufB
-    std::vector<double *> a_phibar, a_gbar, a_phibar_raw, a_h;
+    std::vector<double *> a_phibar, a_gbar, a_phibar_raw, a_h, a_h2;
     double *a_scal = nullptr, *a_chibbar = nullptr, *a_qbar = nullptr, *a_w = nullptr, *a_xbar = nullptr;
+    bool pair_sweeps() const;
     int ensure_adjoint();
     int ensure_adjoint_misc();
     int store_chains(int m, bool compose, const double **gb0);
