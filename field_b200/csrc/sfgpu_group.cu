@@ -154,34 +154,46 @@ __global__ void __launch_bounds__(kThreads, 1) group_diis_kernel(GroupArgs a) {
                 // (sfnewton.cpp:624-628), then the new row: the Gram entries
                 // (i, j) of the kd kept steps, oldest first
                 if (it >= m) {
-                    double e[kHist * kHist / 32];
-#pragma unroll
-                    for (int q = 0; q < kHist * kHist / 32; q++) {
-                        const int idx = lane + 32 * q, i = idx / kHist, j = idx % kHist;
-                        e[q] = (i + 1 < m && j + 1 < m) ? sh.gram[m * (i + 1) + j + 1] : 0.0;
+                    // row by row: row i takes row i + 1, shifted by a column
+#pragma unroll 1
+                    for (int i = 0; i + 1 < m; i++) {
+                        const double v = (lane + 1 < m) ? sh.gram[m * (i + 1) + lane + 1] : 0.0;
+                        __syncwarp();
+                        if (lane + 1 < m) sh.gram[m * i + lane] = v;
+                        __syncwarp();
                     }
-                    __syncwarp();
-#pragma unroll
-                    for (int q = 0; q < kHist * kHist / 32; q++) {
-                        const int idx = lane + 32 * q, i = idx / kHist, j = idx % kHist;
-                        if (i + 1 < m && j + 1 < m) sh.gram[m * i + j] = e[q];
-                    }
-                    __syncwarp();
                 }
                 if (lane < kd) sh.gram[lane + m * (kd - 1)] = sh.gram[kd - 1 + m * lane] = sh.val[lane];
                 __syncwarp();
-                for (int e = lane; e < kd * kd; e += 32) sh.A[e] = sh.gram[(e % kd) + m * (e / kd)];
+                // until the memory is full the oldest step's own product is
+                // 0 (the first step's is never formed, sfnewton.cpp:602-628):
+                // that row goes last in the elimination
+                const int first = (kd > 1 && sh.gram[0] == 0) ? 1 : 0;
+#pragma unroll 1
+                for (int e = lane; e < kd * kd; e += 32) {
+                    const int i = (e / kd + first) % kd, j = (e % kd + first) % kd;
+                    sh.A[e] = sh.gram[i + m * j];
+                }
                 __syncwarp();
-                if (!coeff_ldl_warp(kd, sh.A, sh.coef)) sfb::diis_coeff_warp(kd, sh.A, sh.Q, sh.coef);
-                if (lane == 0) {
-                    double nc = 0;
-                    for (int i = 0; i < kd; i++) nc += sh.coef[i];
-                    for (int i = 0; i < kd; i++) {
-                        sh.coef[i] = sh.coef[i] / nc;
-                        int posi = k - kd + 1 + i;
-                        if (posi < 0) posi += m;
-                        sh.pos[i] = posi;
-                    }
+                const bool ok = coeff_ldl_warp(kd, sh.A, sh.Q, sh.work);
+                __syncwarp();
+                if (ok) {
+                    if (lane < kd) sh.coef[(lane + first) % kd] = sh.Q[lane];
+                    __syncwarp();
+                } else {
+                    for (int e = lane; e < kd * kd; e += 32) sh.A[e] = sh.gram[(e % kd) + m * (e / kd)];
+                    __syncwarp();
+                    sfb::diis_coeff_warp(kd, sh.A, sh.Q, sh.coef);
+                }
+                double nc = 0;
+#pragma unroll 1
+                for (int i = 0; i < kd; i++) nc += sh.coef[i];
+                __syncwarp();
+                if (lane < kd) {
+                    sh.coef[lane] = sh.coef[lane] / nc;
+                    int posi = k - kd + 1 + lane;
+                    if (posi < 0) posi += m;
+                    sh.pos[lane] = posi;
                 }
             }
             __syncthreads();

@@ -42,7 +42,7 @@ struct GShared {
     double val[kVals];
     MolScal scal[sfb::kMaxMol];
     double phib[SFGPU_MAX_SEG], chib[SFGPU_MAX_SEG];
-    double gram[kHist * kHist], A[kHist * kHist], Q[kHist * kHist], coef[kHist];
+    double gram[kHist * kHist], A[kHist * kHist], Q[kHist * kHist], coef[kHist], work[kHist];
     int pos[kHist];
     int inst;
     unsigned long long mbar[2];             // halo rows arrived, by buffer of the running slice
@@ -721,6 +721,12 @@ __device__ __noinline__ void chain1d(const InstDesc &I, int m, double *line, dou
     c.store(c.v, I.ginv0);
 }
 
+// One copy of the logarithm and of the exponential in a kernel whose phases run
+// once an evaluation: such code is bound by instruction fetches, and the
+// functions are called from a dozen places.
+__device__ __noinline__ double log1(double v) { return log(v); }
+__device__ __noinline__ double exp1(double v) { return exp(v); }
+
 // ---- lnGN sums -------------------------------------------------------------
 // Partial sums of w * g over 256-element blocks of the lattice vector, each in
 // the order of wsum_partial's shared-memory tree, into part[0 .. ceil(M/256)).
@@ -750,9 +756,9 @@ __device__ __forceinline__ void wsum_blocks(int M, const double *g, const double
 }
 
 // mol_scalars (sfgpu_kernels.cuh) for a first-order molecule
-__device__ __forceinline__ MolScal mol_scalars_of(const IMol &o, const MolScal *scal, int m, int nmol, double wsum) {
+__device__ __noinline__ MolScal mol_scalars_of(const IMol &o, const MolScal *scal, int m, int nmol, double wsum) {
     MolScal s;
-    s.lngn = log(wsum);
+    s.lngn = log1(wsum);
     double phib = o.phibulk;
     if (o.solvent) {
         phib = 1.0;
@@ -760,18 +766,18 @@ __device__ __forceinline__ MolScal mol_scalars_of(const IMol &o, const MolScal *
             if (q != m) phib -= scal[q].phibulk;
     }
     const double N = (double)o.N;
-    const double gn = exp(s.lngn);
+    const double gn = exp1(s.lngn);
     if (o.freedom == SFGPU_MOL_RESTRICTED) {
-        if (o.type == 0) { s.lnc = log(o.theta) - s.lngn; s.norm = o.theta / gn; }
+        if (o.type == 0) { s.lnc = log1(o.theta) - s.lngn; s.norm = o.theta / gn; }
         else {
-            s.lnc = log(o.theta) - s.lngn - log(1.0 * o.N);
+            s.lnc = log1(o.theta) - s.lngn - log1(1.0 * o.N);
             s.norm = (o.sym ? 2 * o.theta / N : o.theta / N) / gn;
         }
         s.phibulk = o.theta / gn;
     } else {
         s.phibulk = phib;
-        if (o.type == 0) { s.lnc = log(phib); s.norm = phib; }
-        else { s.lnc = log(phib / N); s.norm = o.sym ? 2 * phib / N : phib / N; }
+        if (o.type == 0) { s.lnc = log1(phib); s.norm = phib; }
+        else { s.lnc = log1(phib / N); s.norm = o.sym ? 2 * phib / N : phib / N; }
     }
     if (o.pinned) s.phibulk = 0;
     return s;
@@ -834,25 +840,22 @@ __device__ inline void scalars_group(const InstDesc &I, const Grp &gr, GShared &
     __syncthreads();
 }
 
-// f of one site from its total volume fraction, contact averages and the
-// classes' G (the sums of residual in sfgpu_kernels.cuh, in its order)
-template <class GF>
-__device__ __forceinline__ void put_residual(const InstDesc &I, const double *chib, double phit, const double *rho,
-                                             GF &&gfull, double *f) {
+// f of one site from its total volume fraction, contact averages (by segment)
+// and G (by class): the sums of residual in sfgpu_kernels.cuh, in its order.
+// Rolled loops over local arrays: short code, fetched once.
+__device__ __noinline__ void put_residual(const InstDesc &I, const double *chib, double phit, const double *rho,
+                                          const double *g, double *f) {
     const int ncl = I.nclass, nseg = I.nseg;
     double u[sfb::kResMax];
     double av = 0;
-#pragma unroll
-    for (int c = 0; c < sfb::kResMax; c++) {
-        u[c] = 0;
-        if (c >= ncl) continue;
-        const int st = I.rep[c];
-        double v = -log(gfull(st));
+#pragma unroll 1
+    for (int c = 0; c < ncl; c++) {
+        const double *chi = I.ct.chi + I.rep[c] * SFGPU_MAX_SEG;
+        double v = -log1(g[c]);
         double ci = 0;
-#pragma unroll
-        for (int i = 0; i < sfb::kResMax; i++) {
-            if (i >= nseg) continue;
-            const double xx = I.ct.chi[st * SFGPU_MAX_SEG + i];
+#pragma unroll 1
+        for (int i = 0; i < nseg; i++) {
+            const double xx = chi[i];
             if (xx != 0) ci += xx * rho[i];
         }
         v -= ci / phit;
@@ -861,9 +864,49 @@ __device__ __forceinline__ void put_residual(const InstDesc &I, const double *ch
         av += v;
     }
     av /= ncl;
+    const double t = -1.0 + 1.0 / phit;
+#pragma unroll 1
+    for (int c = 0; c < ncl; c++) f[c] = t + u[c] - av;
+}
+
+// f on a thread's strip; NS bounds the segment types and classes.  Every load of
+// a site is issued before the first use (a segment that is not there or does
+// not interact reads its neighbour in the list again).
+template <int J, bool kCyl, int NS>
+__device__ __noinline__ void sites_residual2d(const InstDesc &I, double *f, const Strip<J> &st, const double *chib) {
+    const DLat &L = I.L;
+    const int nseg = I.nseg, ncl = I.nclass, MY = st.MY;
+    const int dl = (st.k == 1) ? L.map_lo[1] - 1 : -1, dr = (st.k == MY - 2) ? L.map_hi[1] - st.k : 1;
+    const double l = L.l1chi;
+    for (int j = 0; j < st.valid; j++) {
+        const int x = st.x + j, z = st.site + j * MY;
+        const int jj = I.jall[z];
+        const int du = (lat_mapc(L, 0, x - 1) - x) * MY, dd = (lat_mapc(L, 0, x + 1) - x) * MY;
+        const double lm = kCyl ? L.lam_m[x] : l, lp = kCyl ? L.lam_p[x] : l;
+        double e[NS][5], g[NS];
 #pragma unroll
-    for (int c = 0; c < sfb::kResMax; c++)
-        if (c < ncl) f[c] = -1.0 + 1.0 / phit + u[c] - av;
+        for (int i = 0; i < NS; i++) {
+            const double *p = I.phi[min(i, nseg - 1)];
+            e[i][0] = p[z];
+            e[i][1] = p[z + dl];
+            e[i][2] = p[z + dr];
+            e[i][3] = p[z + du];
+            e[i][4] = p[z + dd];
+        }
+#pragma unroll
+        for (int c = 0; c < NS; c++) g[c] = I.gfull[I.rep[min(c, ncl - 1)]][z];
+        double phit = 0, rho[NS];
+#pragma unroll
+        for (int i = 0; i < NS; i++) {
+            const double b = e[i][0], a = e[i][1], c = e[i][2], u = e[i][3], d = e[i][4];
+            if (i < nseg) phit += b;
+            double v;
+            if (kCyl) v = b + lp * (d - b) + lm * (u - b) + l * (a + c - b - b);
+            else v = (1 - 2 * l - lm - lp) * b + l * (u + d) + l * (a + c);
+            rho[i] = (i < nseg && ((I.need >> i) & 1)) ? v : 0.0;
+        }
+        if (jj >= 0) put_residual(I, chib, phit, rho, g, f + (size_t)jj * ncl);
+    }
 }
 
 // ---- x -> f (SF_Solve::residuals, SF_Solve.cpp:647-651) ----------------------
@@ -896,7 +939,7 @@ __device__ inline void residual2d(const InstDesc &I, const double *x, double *f,
             for (int j = 0; j < J; j++) {
                 if (j >= st.valid) continue;
                 const int z = st.site + j * st.MY;
-                const double v = (jx[j] >= 0) ? exp(-xv[j]) : 0.0;
+                const double v = (jx[j] >= 0) ? exp1(-xv[j]) : 0.0;
                 gf[z] = v;
                 if (fr == SFGPU_SEG_PINNED) gs[z] = range[z] > 0 ? v : 0.0;
             }
@@ -968,31 +1011,8 @@ __device__ inline void residual2d(const InstDesc &I, const double *x, double *f,
             }
         }
     }
-    const int up_lo = (L.map_lo[1] - 1), dn_hi = (L.map_hi[1] - (L.Md[1] - 2));
-    const int dl = (st.k == 1) ? up_lo : -1, dr = (st.k == L.Md[1] - 2) ? dn_hi : 1;
-    const double l = L.l1chi;
-    for (int j = 0; j < st.valid; j++) {
-        const int xx = st.x + j, z = st.site + j * st.MY;
-        const int jj = I.jall[z];
-        const int du = (lat_mapc(L, 0, xx - 1) - xx) * st.MY, dd = (lat_mapc(L, 0, xx + 1) - xx) * st.MY;
-        const double lm = kCyl ? L.lam_m[xx] : l, lp = kCyl ? L.lam_p[xx] : l;
-        double phit = 0, rho[sfb::kResMax];
-#pragma unroll
-        for (int i = 0; i < sfb::kResMax; i++) {
-            rho[i] = 0;
-            if (i >= nseg) continue;
-            const double *p = I.phi[i];
-            const double b = p[z];
-            phit += b;
-            if (!((I.need >> i) & 1)) continue;
-            const double a = p[z + dl], c = p[z + dr];
-            const double u = p[z + du], d = p[z + dd];
-            if (kCyl) rho[i] = b + lp * (d - b) + lm * (u - b) + l * (a + c - b - b);
-            else rho[i] = (1 - 2 * l - lm - lp) * b + l * (u + d) + l * (a + c);
-        }
-        if (jj < 0) continue;
-        put_residual(I, sh.chib, phit, rho, [&](int s) { return I.gfull[s][z]; }, f + (size_t)jj * ncl);
-    }
+    if (nseg <= 4 && ncl <= 4) sites_residual2d<J, kCyl, 4>(I, f, st, sh.chib);
+    else sites_residual2d<J, kCyl, sfb::kResMax>(I, f, st, sh.chib);
 }
 
 // where a 1D system's arrays lie (localize1d)
@@ -1011,7 +1031,7 @@ __device__ inline void residual1d(const InstDesc &I, const double *x, double *f,
         const int j = I.jall[r];
         for (int i = 0; i < nseg; i++) {
             if (I.freedom[i] == SFGPU_SEG_FROZEN) continue;
-            const double v = (j >= 0) ? exp(-x[(size_t)j * ncl + I.class_of[i]]) : 0.0;
+            const double v = (j >= 0) ? exp1(-x[(size_t)j * ncl + I.class_of[i]]) : 0.0;
             I.gfull[i][r] = v;
             if (I.freedom[i] == SFGPU_SEG_PINNED) I.gseg[i][r] = I.range[i][I.smap[r]] > 0 ? v : 0.0;
         }
@@ -1068,20 +1088,20 @@ __device__ inline void residual1d(const InstDesc &I, const double *x, double *f,
     for (int z = threadIdx.x + 1; z < M - 1; z += blockDim.x) {
         const int jj = I.jall[z];
         if (jj < 0) continue;
-        double phit = 0, rho[sfb::kResMax];
-#pragma unroll
-        for (int i = 0; i < sfb::kResMax; i++) {
-            rho[i] = 0;
-            if (i >= nseg) continue;
+        double phit = 0, rho[sfb::kResMax], g[sfb::kResMax];
+#pragma unroll 1
+        for (int i = 0; i < nseg; i++) {
             const double *p = I.phi[i];
-            const double b = p[z];
+            const double a = p[z - 1], b = p[z], c = p[z + 1];
             phit += b;
-            if (!((I.need >> i) & 1)) continue;
-            const double a = p[z - 1], c = p[z + 1];
-            if (kCurved) rho[i] = b + L.lamc_p[z] * (c - b) + L.lamc_m[z] * (a - b);
-            else rho[i] = b + l * (a - b - b + c);
+            double v;
+            if (kCurved) v = b + L.lamc_p[z] * (c - b) + L.lamc_m[z] * (a - b);
+            else v = b + l * (a - b - b + c);
+            rho[i] = ((I.need >> i) & 1) ? v : 0.0;
         }
-        put_residual(I, sh.chib, phit, rho, [&](int s) { return I.gfull[s][z]; }, f + (size_t)jj * ncl);
+#pragma unroll 1
+        for (int c = 0; c < ncl; c++) g[c] = I.gfull[I.rep[c]][z];
+        put_residual(I, sh.chib, phit, rho, g, f + (size_t)jj * ncl);
     }
 }
 
@@ -1184,46 +1204,46 @@ __device__ inline void write_back1d(const InstDesc &I, const InstDesc *src, cons
 }
 
 // ---- DIIS coefficients --------------------------------------------------------
-// c = A^-1 1 for the symmetric positive definite Gram matrix by an LDL^T
-// elimination of the augmented system in one warp: lane i holds row i, step k
-// takes one division and one rank-one update where the Jacobi rotations of
-// diis_coeff_warp take n (n - 1) / 2 serial square roots and divisions a
-// sweep.  Returns false, with c unset, when a pivot has lost all but 1e-10 of
-// its diagonal entry (or is not positive): the stored steps are then linearly
-// dependent to rounding and the eigen-decomposition's pseudo-inverse decides.
-__device__ __forceinline__ bool coeff_ldl_warp(int n, const double *A, double *c) {
-    const unsigned full = 0xffffffffu;
+// c = A^-1 1 for the symmetric Gram matrix by eliminating the augmented system
+// in one warp: per column one division a row and a rank-one update shared by
+// the lanes, where the Jacobi rotations of diis_coeff_warp take n (n - 1) / 2
+// serial square roots and divisions a sweep (m = 10: 400 k cycles a call; 8 k
+// here).  The loops stay rolled on purpose: this runs once an iteration, and
+// unrolled over registers it took 50 k cycles, nearly all of them instruction
+// fetches.  A is n x n in shared memory, overwritten; c and w hold n values.
+// Returns false, with c unset, when a pivot keeps less than 1e-14 of the terms
+// it is the sum of: down to there the Gram matrix's own rounding limits either
+// method alike, below it the stored steps are linearly dependent to rounding
+// and the eigen-decomposition's pseudo-inverse decides.
+__device__ __noinline__ bool coeff_ldl_warp(int n, double *A, double *c, double *w) {
     const int lane = threadIdx.x & 31;
-    double a[kHist], rhs = 1.0;
-#pragma unroll
-    for (int j = 0; j < kHist; j++) a[j] = (lane < n && j < n) ? A[lane * n + j] : 0.0;
-    const double diag = (lane < n) ? A[lane * n + lane] : 1.0;
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < kHist; k++) {
-        if (k >= n) break;
-        const double piv = __shfl_sync(full, a[k], k), d0 = __shfl_sync(full, diag, k);
-        if (!(piv > 1e-10 * d0)) { ok = false; break; }
-        const double mul = (lane > k) ? a[k] / piv : 0.0;
-        const double rk = __shfl_sync(full, rhs, k);
-        rhs -= mul * rk;
-#pragma unroll
-        for (int j = k + 1; j < kHist; j++) {
-            if (j >= n) break;
-            const double p = __shfl_sync(full, a[j], k);
-            a[j] -= mul * p;
+    double mag = (lane < n) ? fabs(A[lane * n + lane]) : 0.0;   // of the terms of this row's pivot
+    double rhs = 1.0;                       // row `lane` of the right-hand side
+#pragma unroll 1
+    for (int k = 0; k < n; k++) {
+        const double piv = A[k * n + k];
+        if (!(fabs(piv) > 1e-14 * __shfl_sync(0xffffffffu, mag, k))) return false;
+        const double mul = (lane > k && lane < n) ? A[lane * n + k] / piv : 0.0;
+        rhs -= mul * __shfl_sync(0xffffffffu, rhs, k);
+        if (lane < n) {
+            w[lane] = mul;
+            mag += fabs(mul * A[k * n + lane]);
         }
+        __syncwarp();
+        // the trailing block: half a warp a row
+        const int j = k + 1 + (lane & 15);
+        if (j < n) {
+            const double p = A[k * n + j];
+#pragma unroll 1
+            for (int i = k + 1 + (lane >> 4); i < n; i += 2) A[i * n + j] -= w[i] * p;
+        }
+        __syncwarp();
     }
-    if (!ok) return false;
-    // back substitution: lane k's unknown, then its column out of the rows above
-#pragma unroll
-    for (int k = kHist - 1; k >= 0; k--) {
-        if (k >= n) continue;
-        double xk = 0;
-        if (lane == k) xk = rhs / a[k];
-        xk = __shfl_sync(full, xk, k);
-        if (lane == k) c[k] = xk;
-        if (lane < k) rhs -= a[k] * xk;
+#pragma unroll 1
+    for (int k = n - 1; k >= 0; k--) {
+        const double x = __shfl_sync(0xffffffffu, rhs, k) / A[k * n + k];
+        if (lane == 0) c[k] = x;
+        if (lane < k) rhs -= A[lane * n + k] * x;
     }
     __syncwarp();
     return true;
