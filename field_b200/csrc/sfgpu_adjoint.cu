@@ -204,6 +204,8 @@ int sfgpu_system::ensure_adjoint() {
             sfgpu_set_error(e, "cudaMalloc (dendrimer tree slices)", __FILE__, __LINE__);
             return SFGPU_ERR_NOMEM;
         }
+        // steps write interior sites only; surface layers are read in place as 0
+        SFGPU_CUDA_TRY(cudaMemset(a_dend_gi, 0, sizeof(double) * dend_need));
         a_dend_gi_doubles = dend_need;
     }
     // branched molecules: the cotangents of every U, Q, D slice and a pool
@@ -322,8 +324,7 @@ void sfgpu_system::adj_fstep(const HMol &o, int t, const double *src, double *ds
                                                           nullptr, nullptr, COMP_NONE, 0,
                                                           last ? STEP2_ISO : STEP2_STIFF);
     } else if (K == 6)
-        step2_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst,
-                                                          nullptr, nullptr, COMP_NONE, 0);
+        launch_step2(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
     else
         launch_step2l(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
 }
@@ -343,8 +344,7 @@ void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *ds
                                                           first ? 0.2 : pf[sg * nseg + o.seg[t + 2]], dst, other,
                                                           phi, mode, 1, first ? STEP2_ISO : STEP2_STIFF);
     } else if (K == 6)
-        step2_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst,
-                                                          other, phi, mode, 1);
+        launch_step2(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
     else
         launch_step2l(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
 }

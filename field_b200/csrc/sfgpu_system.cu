@@ -84,6 +84,17 @@ int sfgpu_system::launch_step1(const double *gin, const double *G, double *gout,
     return SFGPU_OK;
 }
 
+// plain second-order 3D step; composing steps are backward ones
+int sfgpu_system::launch_step2(const double *gin, const double *G, double S, double *gout, const double *other,
+                               double *phi, int mode, int backward) {
+    const DLat &L = H.L;
+    const dim3 grid((L.Md[2] - 2 + 31) / 32, (L.Md[1] - 2 + kS2Y - 1) / kS2Y, (L.Md[0] - 2 + kS2X - 1) / kS2X);
+    auto k = !backward ? step2_sites<false, false> : mode == COMP_ACC ? step2_sites<true, true> : step2_sites<true, false>;
+    const cudaError_t e = launch_pdl(k, grid, dim3(32, kS2Y, kS2X), stream, L, gin, G, S, gout, other, phi);
+    if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
+    return SFGPU_OK;
+}
+
 // lumped second-order step: step2l_sites, except at S = 0 or 1, where a weight
 // vanishes that it takes as nonzero
 int sfgpu_system::launch_step2l(const double *gin, const double *G, double S, double *gout, const double *other,
@@ -1312,9 +1323,7 @@ int sfgpu_system::molecule_phi(int m) {
                        (const double *)nullptr, (double *)nullptr, (int)COMP_NONE, 0,
                        (int)(last ? STEP2_ISO : STEP2_STIFF));
         } else if (K == 6)
-            launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg],
-                       pf[o.seg[t - 1] * nseg + sg], out, (const double *)nullptr, (double *)nullptr, (int)COMP_NONE, 0,
-                       (int)STEP2_PLAIN);
+            launch_step2(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
         else
             launch_step2l(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
     };
@@ -1334,8 +1343,7 @@ int sfgpu_system::molecule_phi(int m) {
             launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg], Sv, out, gf,
                        o.d_phi[sg], (int)COMP_ACC, 1, (int)(first ? STEP2_ISO : STEP2_STIFF));
         } else if (K == 6)
-            launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg],
-                       pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], (int)COMP_ACC, 1, (int)STEP2_PLAIN);
+            launch_step2(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
         else
             launch_step2l(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
     };
@@ -2013,9 +2021,7 @@ extern "C" int sfgpu_profile_propagator(sfgpu_system *s, int reps, double *ms_fw
         if (K == 1)
             s->launch_step1(s->d_gi + (t - 1) * KM, G, s->d_gi + t * KM, nullptr, nullptr, COMP_NONE);
         else
-            launch_pdl(step2_rows, dim3(grid_rows(s->H.L)), dim3(kBlock), s->stream, s->H.L,
-                       (const double *)(s->d_gi + (t - 1) * KM), G, 0.2, s->d_gi + t * KM, (const double *)nullptr,
-                       (double *)nullptr, (int)COMP_NONE, 0, (int)STEP2_PLAIN);
+            s->launch_step2(s->d_gi + (t - 1) * KM, G, 0.2, s->d_gi + t * KM, nullptr, nullptr, COMP_NONE, 0);
     }
     SFGPU_CUDA_TRY(cudaEventRecord(e1, s->stream));
     for (int r = 0; r < reps; r++) {
@@ -2025,8 +2031,7 @@ extern "C" int sfgpu_profile_propagator(sfgpu_system *s, int reps, double *ms_fw
         if (K == 1)
             s->launch_step1(src, G, dst, s->d_gi + t * KM, phi, COMP_ACC);
         else
-            launch_pdl(step2_rows, dim3(grid_rows(s->H.L)), dim3(kBlock), s->stream, s->H.L, src, G, 0.2, dst,
-                       (const double *)(s->d_gi + t * KM), phi, (int)COMP_ACC, 1, (int)STEP2_PLAIN);
+            s->launch_step2(src, G, 0.2, dst, s->d_gi + t * KM, phi, COMP_ACC, 1);
     }
     SFGPU_CUDA_TRY(cudaEventRecord(e2, s->stream));
     SFGPU_CUDA_TRY(cudaEventSynchronize(e2));

@@ -155,6 +155,8 @@ struct sfgpu_system {
     int vjp_async(const double *x, const double *w, double *f, double *xbar);
     int launch_step1_t(const double *gin, const double *dgin, const double *G, const double *dG, double *gout,
                        double *dgout, const double *other, const double *dother, double *phi, double *dphi, int mode);
+    int launch_step2(const double *gin, const double *G, double S, double *gout, const double *other, double *phi,
+                     int mode, int backward);
     int launch_step2l(const double *gin, const double *G, double S, double *gout, const double *other, double *phi,
                       int mode, int backward);
     int launch_step1(const double *gin, const double *G, double *gout, const double *other, double *phi, int mode);
