@@ -243,7 +243,7 @@ static __global__ void __launch_bounds__(128) adj_gather_sites(DLat L, AdjPair p
 
 // the same on the six-neighbour 3D lattices, in the columns of step3d_cols
 template <bool kStart>
-__device__ __forceinline__ void adj_cols(const DLat &L, const AdjStep &o, const Column &c) {
+__device__ __forceinline__ void adj_cols(const DLat &L, const AdjStep &o, const Column<> &c) {
     const int nx = L.Md[0] - 2;
     const int z = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * kColY + threadIdx.y + 1;
     const double s6 = 1.0 / 6.0;
@@ -285,14 +285,14 @@ __device__ __forceinline__ void adj_cols(const DLat &L, const AdjStep &o, const 
 template <bool kStart>
 static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols(DLat L, AdjStep o) {
     sfk::pdl_enter();
-    const Column c(L);
+    const Column<> c(L);
     if (c.in) adj_cols<kStart>(L, o, c);
 }
 template <bool kStart>
 static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols_pair(DLat L, AdjPair p, int nzb) {
     sfk::pdl_enter();
     const int q = blockIdx.z >= nzb;
-    Column c(L);
+    Column<> c(L);
     if (!c.in) return;
     c.x0 -= q * nzb * kCols;
     adj_cols<kStart>(L, p.s[q], c);

@@ -281,7 +281,10 @@ bool group_shape(const sfgpu_system *s, int blocks, int threads, int m, GroupSha
         const int n = L.Md[0] - 2;
         g.C = 1;
         g.J = 1;
-        g.threads = std::max(128, 32 * warps1d(n));
+        // the phases between the chains want a thread per site (one system alone,
+        // n = 200: 3.30 ms a solve with 128 threads, 2.95 with 256); two blocks
+        // share an SM in a large batch, whose registers then hold 128 each
+        g.threads = std::max(blocks > 1 ? 256 : 128, 32 * warps1d(n));
         // what localize1d takes, in its order; the last ones only where they fit
         size_t chain = 0;
         int nonfrozen = 0, pinned = 0, molphis = 0;

@@ -417,13 +417,14 @@ step3d_march_pf2(DLat L, const double *__restrict__ gin, const double *__restric
 // 10-40 % (registers), blocks of eight rows 5 %.  Operands and order as
 // step3d_march: bit-identical.
 constexpr int kCols = 4, kColY = 4;
-struct Column {              // a thread's columns: site of plane x is x * jx + col
+template <int U = kCols>
+struct Column {              // a thread's U columns: site of plane x is x * jx + col
     int x0, col, oy[2], oz[2];
     bool in;
     __device__ __forceinline__ Column(const DLat &L) {
         const int ny = L.Md[1] - 2, nz = L.Md[2] - 2;
         const int z = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * kColY + threadIdx.y + 1;
-        x0 = blockIdx.z * kCols + 1;
+        x0 = blockIdx.z * U + 1;
         in = z <= nz && y <= ny;
         col = y * L.st[1] + z;
         oy[0] = (lat_mapc(L, 1, y - 1) - y) * L.st[1];
@@ -431,18 +432,18 @@ struct Column {              // a thread's columns: site of plane x is x * jx + 
         oz[0] = lat_mapc(L, 2, z - 1) - z;
         oz[1] = lat_mapc(L, 2, z + 1) - z;
     }
-    // the column's values at planes x0 - 1 .. x0 + kCols
-    __device__ __forceinline__ void planes(const DLat &L, const double *__restrict__ p, double (&v)[kCols + 2]) const {
+    // the column's values at planes x0 - 1 .. x0 + U
+    __device__ __forceinline__ void planes(const DLat &L, const double *__restrict__ p, double (&v)[U + 2]) const {
 #pragma unroll
-        for (int u = 0; u < kCols + 2; u++)
+        for (int u = 0; u < U + 2; u++)
             v[u] = (x0 - 1 + u < L.Md[0]) ? p[lat_mapc(L, 0, x0 - 1 + u) * L.st[0] + col] : 0.0;
     }
     __device__ __forceinline__ void sides(const double *__restrict__ p, int t, double (&a)[4]) const {
         a[0] = p[t + oy[0]]; a[1] = p[t + oy[1]]; a[2] = p[t + oz[0]]; a[3] = p[t + oz[1]];
     }
 };
-inline dim3 cols_grid(const DLat &L) {
-    return dim3((L.Md[2] - 2 + 31) / 32, (L.Md[1] - 2 + kColY - 1) / kColY, (L.Md[0] - 2 + kCols - 1) / kCols);
+inline dim3 cols_grid(const DLat &L, int planes = kCols) {
+    return dim3((L.Md[2] - 2 + 31) / 32, (L.Md[1] - 2 + kColY - 1) / kColY, (L.Md[0] - 2 + planes - 1) / planes);
 }
 
 template <int kMode>
@@ -450,7 +451,7 @@ static __global__ void __launch_bounds__(32 * kColY, 6)
 step3d_cols(DLat L, const double *__restrict__ gin, const double *__restrict__ G, double *__restrict__ gout,
             const double *__restrict__ other, double *__restrict__ phi) {
     pdl_enter();
-    const Column c(L);
+    const Column<> c(L);
     if (!c.in) return;
     const int nx = L.Md[0] - 2;
     double v[kCols + 2], a[kCols][4], g[kCols], ot[kCols], ph[kCols];
@@ -497,7 +498,7 @@ static __global__ void __launch_bounds__(128) step1_sites_pair(DLat L, PairStep 
 static __global__ void __launch_bounds__(32 * kColY, 6) step3d_cols_pair(DLat L, PairStep p, int nz) {
     pdl_enter();
     const int q = blockIdx.z >= nz;
-    Column c(L);
+    Column<> c(L);
     if (!c.in) return;
     c.x0 -= q * nz * kCols;
     const int nx = L.Md[0] - 2;

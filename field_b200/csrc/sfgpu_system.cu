@@ -763,6 +763,7 @@ int sfgpu_system::setup_group() {
         for (const auto &o : mols)
             if (o.d_phi[i]) SFGPU_CUDA_TRY(cudaMemset(o.d_phi[i], 0, sizeof(double) * M));
     }
+    std::vector<int>().swap(jmap_h);
     group = true;
     return SFGPU_OK;
 }

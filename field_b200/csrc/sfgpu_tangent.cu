@@ -83,7 +83,7 @@ int sfgpu_system::launch_step1_t(const double *gin, const double *dgin, const do
     if (L.grad == 3 && !lat_twelve(L)) {
         auto k = mode == COMP_ACC ? step3d_cols_t<COMP_ACC>
                                   : mode == COMP_CENTRE ? step3d_cols_t<COMP_CENTRE> : step3d_cols_t<COMP_NONE>;
-        e = launch_pdl(k, cols_grid(L), dim3(32, kColY), stream, L, gin, dgin, G, dG, gout, dgout, other, dother, phi, dphi);
+        e = launch_pdl(k, cols_grid(L, kColsT), dim3(32, kColY), stream, L, gin, dgin, G, dG, gout, dgout, other, dother, phi, dphi);
     } else if (L.grad < 3) {
         e = launch_pdl(step1_sites_t, sites_grid(L), sites_block(L), stream, L, gin, dgin, G, dG, gout, dgout, other,
                        dother, phi, dphi, mode);

@@ -119,24 +119,26 @@ step1_sites_t(DLat L, const double *__restrict__ gin, const double *__restrict__
     });
 }
 
-// step1_rows_t on the six-neighbour 3D lattices, in the columns of
-// step3d_cols: 90 x 75 x 61, 13.5 us a step by rows, 5.9 this way.
+// step1_rows_t on the six-neighbour 3D lattices, in columns as step3d_cols: two
+// planes a thread, as twice the fields take the registers of four.  J v on
+// 90 x 75 x 61, N = 64: 1757 us by rows, 1117 with four planes, 958 with two.
 // Same operands and order, bit-identical.
+constexpr int kColsT = 2;
 template <int kMode>
-static __global__ void __launch_bounds__(32 * kColY, 4)
+static __global__ void __launch_bounds__(32 * kColY, 5)
 step3d_cols_t(DLat L, const double *__restrict__ gin, const double *__restrict__ dgin, const double *__restrict__ G,
               const double *__restrict__ dG, double *__restrict__ gout, double *__restrict__ dgout,
               const double *__restrict__ other, const double *__restrict__ dother, double *__restrict__ phi,
               double *__restrict__ dphi) {
     pdl_enter();
-    const Column c(L);
+    const Column<kColsT> c(L);
     if (!c.in) return;
     const int nx = L.Md[0] - 2;
-    double v[kCols + 2], w[kCols + 2];
+    double v[kColsT + 2], w[kColsT + 2];
     c.planes(L, gin, v);
     c.planes(L, dgin, w);
 #pragma unroll
-    for (int u0 = 0; u0 < kCols; u0 += 2) {      // two planes' side loads at a time
+    for (int u0 = 0; u0 < kColsT; u0 += 2) {
         double a[2][4], b[2][4], g[2], dg[2], ot[2], dot[2], ph[2], dp[2];
 #pragma unroll
         for (int e = 0; e < 2; e++) {
