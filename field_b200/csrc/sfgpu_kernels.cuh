@@ -726,17 +726,18 @@ step2_rows(DLat L, const double *__restrict__ gin, const double *__restrict__ G,
 // Block shapes from 32 x 4 x 1 to 32 x 2 x 8 lie within 4 % of one another: the
 // forward step is not held by the reads that neighbours share but by the 45 MB
 // slice it writes to memory beside the one it reads from L2.
+// The offsets and mirror flags are formed before pdl_enter(), while the previous
+// step drains (whole residual, 40 segments, us): 16^3 341 -> 305 (a warp per row
+// 322), 60 x 60 x 40 634 -> 561, 96 x 96 x 16 680 -> 579.
 constexpr int kS2Y = 2, kS2X = 2;
 template <bool kBackward, bool kAcc>
 static __global__ void __launch_bounds__(32 * kS2Y * kS2X)
 step2_sites(DLat L, const double *__restrict__ gin, const double *__restrict__ G, double S, double *__restrict__ gout,
             const double *__restrict__ other, double *__restrict__ phi) {
-    pdl_enter();
     const int M = L.M;
     const int nx = L.Md[0] - 2, ny = L.Md[1] - 2, nz = L.Md[2] - 2;
     const int z = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * kS2Y + threadIdx.y + 1;
     const int x = blockIdx.z * kS2X + threadIdx.z + 1;
-    if (z > nz || y > ny || x > nx) return;
     const int t = x * L.st[0] + y * L.st[1] + z;
     const double Lw = (1.0 - S) / 4.0;
     // by direction: 0 = -x, 1 = +x, 2 = -y, 3 = +y, 4 = -z, 5 = +z
@@ -746,6 +747,8 @@ step2_sites(DLat L, const double *__restrict__ gin, const double *__restrict__ G
     const bool sw[6] = {x == 1 && is_mirror(L.bc_lo[0]), x == nx && is_mirror(L.bc_hi[0]),
                         y == 1 && is_mirror(L.bc_lo[1]), y == ny && is_mirror(L.bc_hi[1]),
                         z == 1 && is_mirror(L.bc_lo[2]), z == nz && is_mirror(L.bc_hi[2])};
+    pdl_enter();
+    if (z > nz || y > ny || x > nx) return;
     const double g = G[t];
     const double gS = g * S, gL = g * Lw;
     double oth[6], ph = 0;
