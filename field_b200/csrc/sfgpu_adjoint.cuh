@@ -228,10 +228,10 @@ struct AdjStep {
 // stored): grid.z, 2D and 1D; the second half of grid.z in 3D
 struct AdjPair { AdjStep s[2]; };
 static __global__ void __launch_bounds__(128) adj_gather_sites(DLat L, AdjPair p) {
-    sfk::pdl_enter();
     const AdjStep &a = p.s[blockIdx.z];
     for_site(L, [&](const RowInfo &R, int k, int nlast) {
         const int t = R.base + k;
+        sfk::pdl_enter();
         const double P = a.P[t], pr = a.pr[t], Q = a.Q[t], H = a.H[t], g = a.G[t];
         double c = pr * P;
         if (a.w) c += *a.qbar * a.w[t];
@@ -284,15 +284,15 @@ __device__ __forceinline__ void adj_cols(const DLat &L, const AdjStep &o, const 
 }
 template <bool kStart>
 static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols(DLat L, AdjStep o) {
-    sfk::pdl_enter();
     const Column<> c(L);
+    sfk::pdl_enter();
     if (c.in) adj_cols<kStart>(L, o, c);
 }
 template <bool kStart>
 static __global__ void __launch_bounds__(32 * kColY, 5) adj_gather_cols_pair(DLat L, AdjPair p, int nzb) {
-    sfk::pdl_enter();
     const int q = blockIdx.z >= nzb;
     Column<> c(L);
+    sfk::pdl_enter();
     if (!c.in) return;
     c.x0 -= q * nzb * kCols;
     adj_cols<kStart>(L, p.s[q], c);

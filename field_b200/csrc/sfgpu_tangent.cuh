@@ -99,9 +99,9 @@ step1_sites_t(DLat L, const double *__restrict__ gin, const double *__restrict__
               const double *__restrict__ dG, double *__restrict__ gout, double *__restrict__ dgout,
               const double *__restrict__ other, const double *__restrict__ dother, double *__restrict__ phi,
               double *__restrict__ dphi, int mode) {
-    pdl_enter();
     for_site(L, [&](const RowInfo &R, int k, int nlast) {
         const int t = R.base + k;
+        pdl_enter();
         double ot = 0, dot = 0, ph = 0, dp = 0;
         if (mode == COMP_ACC) { ot = other[t]; dot = dother[t]; }
         if (mode != COMP_NONE) { ph = phi[t]; dp = dphi[t]; }
@@ -121,7 +121,8 @@ step1_sites_t(DLat L, const double *__restrict__ gin, const double *__restrict__
 
 // step1_rows_t on the six-neighbour 3D lattices, in columns as step3d_cols: two
 // planes a thread, as twice the fields take the registers of four.  J v on
-// 90 x 75 x 61, N = 64: 1757 us by rows, 1117 with four planes, 958 with two.
+// 90 x 75 x 61, N = 64: 1757 us by rows, 1117 with four planes, 958 with two (925 with
+// the offsets formed before pdl_enter()).
 // Same operands and order, bit-identical.
 constexpr int kColsT = 2;
 template <int kMode>
@@ -130,8 +131,8 @@ step3d_cols_t(DLat L, const double *__restrict__ gin, const double *__restrict__
               const double *__restrict__ dG, double *__restrict__ gout, double *__restrict__ dgout,
               const double *__restrict__ other, const double *__restrict__ dother, double *__restrict__ phi,
               double *__restrict__ dphi) {
-    pdl_enter();
     const Column<kColsT> c(L);
+    pdl_enter();
     if (!c.in) return;
     const int nx = L.Md[0] - 2;
     double v[kColsT + 2], w[kColsT + 2];
