@@ -8,10 +8,10 @@ N 20..1000) from x = 0.
 
 One step = one batch of instances solved to convergence.  ``--form chosen``
 runs the batched persistent solver (one launch per batch), ``--form plain``
-the per-instance host-driven form.  The line also carries ``plain_gpu_form``:
-per-instance Pure_DIIS with one launch per propagator step on the cylinder,
-SFbox's own Newton iteration (pseudohessian) over the device residual on the
-1D instances, where its dense Hessian fits.
+the per-instance form.  The line also carries ``plain_gpu_form``:
+Pure_DIIS one instance after another on the cylinder, SFbox's own Newton
+iteration (pseudohessian) over the device residual on the 1D instances, where
+its dense Hessian fits.
 
 ``--impl reference`` times SFbox itself -- the reference's C++ sources built
 by oracle/refbuild (oracle/_ref/sfref) -- on all host cores, one process per
@@ -48,9 +48,6 @@ WORKLOADS = {
                    "chi_AW grid over [0,1], phibulk 1e-4..1e-1, chi_AS -2..0), (A)N + W at a frozen surface, x0 = 0",
            "m": 5, "eta": 0.1, "maxit": 5000},
 }
-# ncu: 93.36 GB read + 76.00 GB written by one batch_diis_kernel launch of
-# 148 cylinder instances that made 148 * (33.63 + 1) residual evaluations
-DRAM_BYTES_PER_INSTANCE_ITERATION_C2 = (93.365e9 + 76.002e9) / (148 * 34.63)
 
 
 def parse():
@@ -403,19 +400,12 @@ def run_ours(a, rank, world, local_rank):
         ns = min(a.plain_sample, len(insts))
         pv, prof_sys, _, pconv = plain_form(cfg, insts[:ns], stream, steps=1)
         plain = {"value": pv, "unit": "solves/s", "instances": ns, "converged": int(pconv),
-                 "form": ("per-instance host-driven Pure_DIIS, one launch per propagator step" if cfg == "c2" else
+                 "form": ("per-instance Pure_DIIS, one launch per solve" if cfg == "c2" else
                           "per-instance SFbox Newton iteration (pseudohessian, Scheutjens step search) "
                           "over the device residual, host-driven")}
         kp_bytes = solver.algorithmic_bytes(last_iters)
-        prof_k = {"kernel": "batch_diis_kernel (persistent, one launch per batch solve)",
+        prof_k = {"kernel": "group_diis_kernel (a cluster per instance, one launch per batch solve)",
                   "bytes": kp_bytes, "ms": statistics.median(kms)}
-        if cfg == "c2":
-            # DRAM traffic measured by ncu (dram__bytes_read.sum +
-            # dram__bytes_write.sum) on one launch of 148 instances of this
-            # workload, per instance and DIIS iteration, scaled to this
-            # launch's iterations
-            prof_k["traffic"] = DRAM_BYTES_PER_INSTANCE_ITERATION_C2 * float(sum(int(i) + 1 for i in last_iters))
-            prof_k["traffic_source"] = "ncu capture of 148 instances, scaled by residual evaluations"
         solver.kernel_profile = prof_k
     prof = prof_sys.profile_propagator(reps=400)
     roof = fbatch.roofline(prof, a.form, solver)

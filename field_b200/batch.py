@@ -29,10 +29,25 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
+def one_launch(spec) -> bool:
+    """Whether the cluster engine evaluates (and iterates) the system in one
+    launch: linear first-order chains on 1D and 2D lattices (group_eligible in
+    csrc/sfgpu_group.cu)."""
+    lat = spec.lattice
+    n = lat.n_layers[:lat.gradients]
+    if lat.order != 1 or lat.gradients > 2 or spec.overflow_protection or spec.charged or min(n) < 3:
+        return False
+    if any(m.generations or m.bond_parent is not None or m.ring or m.force for m in spec.molecules):
+        return False
+    return lat.gradients == 2 or (4 not in (lat.bound_lo[0], lat.bound_hi[0]) and n[0] <= 1664)
+
+
 def launches_per_residual(spec) -> int:
     """Kernel launches of one single-system residual evaluation
     (sfgpu_system::residual_async): SWF updates, per-molecule propagation,
     state sums, bulk scalars and the residual kernel."""
+    if one_launch(spec):
+        return 1
     K = spec.lattice.components
     n = 0
     for s in spec.segments:
@@ -54,8 +69,10 @@ def launches_per_residual(spec) -> int:
 def launch_count(form: str, iterations_total: int, insts, solver=None) -> int:
     if form == "chosen" and solver is not None:
         return solver.launches_in_last_solve_total
-    per = launches_per_residual(insts[0][0])
     n_inst = len(insts)
+    if one_launch(insts[0][0]):
+        return n_inst   # a solve is one launch
+    per = launches_per_residual(insts[0][0])
     # per DIIS iteration: residual + step + dots + sum + combine; plus the start
     return iterations_total * (per + 4) + n_inst * (per + 3)
 
@@ -66,12 +83,12 @@ def roofline(prof: dict, form: str, solver=None) -> dict:
         kp = solver.kernel_profile
         ach = kp["bytes"] / (kp["ms"] / 1e3) / 1e9
         return {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                "traffic": kp.get("traffic"), "traffic_source": kp.get("traffic_source"),
+                "traffic": None,
                 "peak_kind": kind, "kernel": kp["kernel"],
                 "bytes_per_launch": kp["bytes"], "ms_per_launch": kp["ms"]}
     ach = prof["bytes_bwd"] / (prof["ms_bwd"] / 1e3) / 1e9
     return {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": None,
-            "peak_kind": kind, "kernel": "step1 (backward step + fused composition)",
+            "peak_kind": kind, "kernel": "first-order step (backward + fused composition)",
             "bytes_per_launch": prof["bytes_bwd"], "ms_per_launch": prof["ms_bwd"],
             "forward_step": {"bytes": prof["bytes_fwd"], "ms": prof["ms_fwd"],
                              "achieved": prof["bytes_fwd"] / (prof["ms_fwd"] / 1e3) / 1e9}}

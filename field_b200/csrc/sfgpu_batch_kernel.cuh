@@ -1,6 +1,7 @@
 // sfgpu_batch_kernel.cuh -- the persistent batched Pure_DIIS kernel
 // (SFNewton::PlainLBFGSDIIS, sfnewton.cpp:566-664, one instance per thread
-// block).  kWide = false compiles the six-neighbour lattices only (every
+// block; linear chains on 1D and 2D lattices run in the cluster engine,
+// sfgpu_group.cuh).  kWide = false compiles the six-neighbour lattices only (every
 // configuration of the bench) and is instantiated in sfgpu_batch.cu;
 // kWide = true also compiles the FCC, HEX and stencils lattice types and the
 // force ensemble and is instantiated alone in sfgpu_batch_wide.cu, so that

@@ -439,13 +439,13 @@ int sfgpu_profile_propagator(sfgpu_system *sys, int reps, double *ms_fwd, double
  * buffers and keep the fastest (reps forward + backward steps each; the
  * propagator contents are overwritten).  Other lattices ignore it. */
 int sfgpu_system_set_tile(sfgpu_system *sys, int xc);
-/* 1: the 3D first-order step runs software-pipelined (plane x+1's loads in
- * flight while plane x is computed, double-buffered tile); 0: the plain
- * x-marching form; 2: pipelined, the forward (composition-free) steps with
- * two y rows of columns per thread.  Results are bit-identical.  By default
- * the composing backward steps run pipelined (x depth 8) and the forward
- * steps plain (depth 4); the autotuner times the forms and depths for each
- * kind of step.  sfgpu_system_set_tile and this call set both kinds. */
+/* March forms of the 3D first-order step.  1: software-pipelined (plane x+1's
+ * loads in flight while plane x is computed, double-buffered tile); 0: the
+ * plain x-marching form; 2: pipelined, the forward (composition-free) steps
+ * with two y rows of columns per thread.  By default no march runs: a thread
+ * owns four planes of one column.  Results are bit-identical.  The autotuner
+ * times every form, and the marches' depths, for each kind of step.
+ * sfgpu_system_set_tile (which selects a march) and this call set both kinds. */
 int sfgpu_system_set_tile_pipelined(sfgpu_system *sys, int enable);
 int sfgpu_system_autotune(sfgpu_system *sys, int reps, int *chosen_xc, double *best_ms);
 
@@ -520,6 +520,8 @@ int sfgpu_batch_set_stream(sfgpu_batch *batch, void *stream);
  * multiple of 32; default 1024, 512, 384 or 256 by lattice size) and whether G of
  * the running segment (and on 1D symmetric homopolymers the running slices,
  * phi and a ring of stored slices) is staged in shared memory (default 1).
+ * Batches of linear chains on 1D or 2D lattices of one geometry run a
+ * thread-block cluster per instance, whose shape this call leaves as it is.
  * Results do not depend on it; the autotuner of field_b200.batch times the
  * candidates. */
 int sfgpu_batch_set_launch(sfgpu_batch *batch, int threads, int stage);
