@@ -321,8 +321,10 @@ struct Chain2 {
                 if (kFull || j < st.valid) { a[u] = s[j * PW - 1]; c[u] = s[j * PW + 1]; }
                 if (kLamReg) { lm[u] = lmr[j]; lp[u] = lpr[j]; }
                 else if (kCyl) {
-                    lm[u] = dyn_smem()[lam + j];
-                    lp[u] = dyn_smem()[lam + lamrows + j];
+                    // the table ends with the block's rows, the last strip may not
+                    const bool in = kFull || j < st.valid;
+                    lm[u] = in ? dyn_smem()[lam + j] : 0.0;
+                    lp[u] = in ? dyn_smem()[lam + lamrows + j] : 0.0;
                 }
             }
 #pragma unroll
