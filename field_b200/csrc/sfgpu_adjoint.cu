@@ -152,6 +152,8 @@ __global__ void adj_swf(int nsites, SwfAdj sa, const int *__restrict__ sites, do
 }  // namespace
 
 // cotangent vectors and scalars of the reverse sweep (any lattice order)
+// (cleared on the system's stream, as everything here: the default stream is
+// not ordered with it)
 int sfgpu_system::ensure_adjoint_misc() {
     int rc;
     if (!a_misc) {
@@ -166,12 +168,12 @@ int sfgpu_system::ensure_adjoint_misc() {
         if ((rc = alloc_d(&a_cot[0], (size_t)K * M)) || (rc = alloc_d(&a_cot[1], (size_t)K * M))) return rc;
         if (K == 1 && ((rc = alloc_d(&a_cot2[0], M)) || (rc = alloc_d(&a_cot2[1], M)))) return rc;
         if (K == 1) {
-            SFGPU_CUDA_TRY(cudaMemset(a_cot2[0], 0, sizeof(double) * M));
-            SFGPU_CUDA_TRY(cudaMemset(a_cot2[1], 0, sizeof(double) * M));
+            SFGPU_CUDA_TRY(cudaMemsetAsync(a_cot2[0], 0, sizeof(double) * M, stream));
+            SFGPU_CUDA_TRY(cudaMemsetAsync(a_cot2[1], 0, sizeof(double) * M, stream));
         }
         // the gathering steps read surface layers, which no step writes
-        SFGPU_CUDA_TRY(cudaMemset(a_cot[0], 0, sizeof(double) * K * M));
-        SFGPU_CUDA_TRY(cudaMemset(a_cot[1], 0, sizeof(double) * K * M));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_cot[0], 0, sizeof(double) * K * M, stream));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_cot[1], 0, sizeof(double) * K * M, stream));
         if ((rc = alloc_d(&a_scal, sizeof(AdjScal) / sizeof(double) * (size_t)nmol)) || (rc = alloc_d(&a_chibbar, SFGPU_MAX_SEG)) ||
             (rc = alloc_d(&a_qbar, 1)))
             return rc;
@@ -205,7 +207,7 @@ int sfgpu_system::ensure_adjoint() {
             return SFGPU_ERR_NOMEM;
         }
         // steps write interior sites only; surface layers are read in place as 0
-        SFGPU_CUDA_TRY(cudaMemset(a_dend_gi, 0, sizeof(double) * dend_need));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_dend_gi, 0, sizeof(double) * dend_need, stream));
         a_dend_gi_doubles = dend_need;
     }
     // branched molecules: the cotangents of every U, Q, D slice and a pool
@@ -269,7 +271,7 @@ int sfgpu_system::ensure_adjoint() {
         }
         // boundary entries of the slices are read only on surface layers, where
         // propagators are 0: start from zeros
-        SFGPU_CUDA_TRY(cudaMemset(a_store, 0, sizeof(double) * slices * KM));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(a_store, 0, sizeof(double) * slices * KM, stream));
         if (a_stride == 0) {
             a_gf = a_store;
             a_gb = a_store + (size_t)nmax * KM;

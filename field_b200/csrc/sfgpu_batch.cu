@@ -83,7 +83,8 @@ static int configure_stage(sfgpu_batch *b, bool allow) {
         b->desc_h[i].small1d = sym1d ? 1 : 0;
         if (sym1d) need = std::max(need, vecs);
     }
-    if (cudaMemcpy(b->d_desc, b->desc_h.data(), sizeof(InstDesc) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
+    if (cudaMemcpyAsync(b->d_desc, b->desc_h.data(), sizeof(InstDesc) * n, cudaMemcpyHostToDevice, b->stream) !=
+            cudaSuccess ||
         cudaFuncSetAttribute(batch_kernel(b), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) !=
             cudaSuccess)
         return SFGPU_ERR_CUDA;
@@ -212,7 +213,6 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
             break;
     }
     if (!rc) rc = balloc(b, (void **)&b->d_desc, sizeof(InstDesc) * n);
-    if (!rc && cudaMemcpy(b->d_desc, b->desc_h.data(), sizeof(InstDesc) * n, cudaMemcpyHostToDevice) != cudaSuccess) rc = SFGPU_ERR_CUDA;
     if (!rc) rc = balloc(b, (void **)&b->d_queue, sizeof(int));
     if (!rc) rc = balloc(b, (void **)&b->d_status, sizeof(int) * n);
     if (!rc) rc = balloc(b, (void **)&b->d_iters, sizeof(int) * n);
@@ -223,6 +223,7 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
     b->block = maxM >= 4096 ? 1024 : (maxM >= 1024 ? 512 : (maxM >= 384 ? 384 : 256));
     if ((rc = configure_stage(b, true))) { delete b; return rc; }
     configure_group(b);
+    if ((rc = sfgpu_after_setup(b->stream))) { delete b; return rc; }
     *out = b;
     return SFGPU_OK;
 }

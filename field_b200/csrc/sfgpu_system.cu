@@ -809,14 +809,15 @@ int sfgpu_system::solve_group(double *x, double tol, int maxit, int m, double et
         diis_m = 0;
         const int rc = dalloc(&d_diis, nvar * (2 + 2 * (size_t)m) + 1);
         if (rc) { d_diis = nullptr; return rc; }
-        diis_m = m;
         sfb::InstDesc I;
-        SFGPU_CUDA_TRY(cudaMemcpy(&I, d_inst, sizeof(I), cudaMemcpyDeviceToHost));
+        SFGPU_CUDA_TRY(cudaMemcpyAsync(&I, d_inst, sizeof(I), cudaMemcpyDeviceToHost, st));
+        SFGPU_CUDA_TRY(cudaStreamSynchronize(st));
         I.x = d_diis;
         I.g = I.x + nvar;
         I.XR = I.g + nvar;
         I.XX0 = I.XR + nvar * (size_t)m;
-        SFGPU_CUDA_TRY(cudaMemcpy(d_inst_solve, &I, sizeof(I), cudaMemcpyHostToDevice));
+        SFGPU_CUDA_TRY(cudaMemcpyAsync(d_inst_solve, &I, sizeof(I), cudaMemcpyHostToDevice, st));
+        diis_m = m;
     }
     double *err = d_diis + nvar * (2 + 2 * (size_t)diis_m);
     SFGPU_CUDA_TRY(cudaMemcpyAsync(d_diis, x, sizeof(double) * nvar, cudaMemcpyHostToDevice, st));
@@ -1668,6 +1669,16 @@ bool sfgpu_system::primal_checkpointed(const HMol &o) const {
            !logmode;
 }
 
+int sfgpu_after_setup(cudaStream_t stream) {
+    cudaEvent_t e;
+    SFGPU_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    cudaError_t rc = cudaEventRecord(e, cudaStreamLegacy);
+    if (rc == cudaSuccess) rc = cudaStreamWaitEvent(stream, e, 0);
+    cudaEventDestroy(e);
+    SFGPU_CUDA_TRY(rc);
+    return SFGPU_OK;
+}
+
 static int create_system(const sfgpu_system_desc *desc, int stride, sfgpu_system **out) {
     if (!desc || !out) return fail(SFGPU_ERR_INVALID, "null argument");
     if (stride < 0) return fail(SFGPU_ERR_INVALID, "checkpoint stride must be >= 0");
@@ -1683,6 +1694,7 @@ static int create_system(const sfgpu_system_desc *desc, int stride, sfgpu_system
     int rc = s->setup(desc);
     if (!rc) rc = s->setup_group();
     if (!rc && s->group) rc = s->setup_group_single();
+    if (!rc) rc = sfgpu_after_setup(s->stream);
     if (rc) { delete s; return rc; }
     *out = s;
     return SFGPU_OK;

@@ -21,6 +21,12 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Systems are set up by copies and clears on the default stream and run on a
+// stream of their own, which is not ordered with it: what follows on `stream`
+// waits for all of them (a copy from pageable memory may still be on its way
+// when the call returns, a clear always).
+int sfgpu_after_setup(cudaStream_t stream);
+
 struct GroupShape;
 namespace sfb { struct InstDesc; }
 

@@ -33,7 +33,7 @@ int sfgpu_system::ensure_tangent() {
     dgfull.assign(nseg, nullptr); dgseg.assign(nseg, nullptr); dphi.assign(nseg, nullptr);
     for (int i = 0; i < nseg; i++) {
         if ((rc = alloc_d(&dphi[i], M))) return rc;
-        SFGPU_CUDA_TRY(cudaMemset(dphi[i], 0, sizeof(double) * M));   // frozen states: 0
+        SFGPU_CUDA_TRY(cudaMemsetAsync(dphi[i], 0, sizeof(double) * M, stream));   // frozen states: 0
         if (freedom[i] == SFGPU_SEG_FROZEN) continue;
         if ((rc = alloc_d(&dgfull[i], M))) return rc;
         if ((rc = alloc_d(&dgseg[i], M))) return rc;
@@ -56,17 +56,17 @@ int sfgpu_system::ensure_tangent() {
     t_gi = d_gi;
     if (ck) {
         if ((rc = alloc_d(&t_gi, store))) return rc;
-        SFGPU_CUDA_TRY(cudaMemset(t_gi, 0, sizeof(double) * std::max<size_t>(store, 1)));
+        SFGPU_CUDA_TRY(cudaMemsetAsync(t_gi, 0, sizeof(double) * std::max<size_t>(store, 1), stream));
     }
     if ((rc = alloc_d(&t_w[0], (size_t)K * M)) || (rc = alloc_d(&t_w[1], (size_t)K * M))) return rc;
-    SFGPU_CUDA_TRY(cudaMemset(t_w[0], 0, sizeof(double) * K * M));
-    SFGPU_CUDA_TRY(cudaMemset(t_w[1], 0, sizeof(double) * K * M));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(t_w[0], 0, sizeof(double) * K * M, stream));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(t_w[1], 0, sizeof(double) * K * M, stream));
     if ((rc = alloc_d(&d_dginv[0], (size_t)K * M)) || (rc = alloc_d(&d_dginv[1], (size_t)K * M))) return rc;
-    SFGPU_CUDA_TRY(cudaMemset(d_dgi, 0, sizeof(double) * std::max<size_t>(store, 1)));
-    SFGPU_CUDA_TRY(cudaMemset(d_dginv[0], 0, sizeof(double) * K * M));
-    SFGPU_CUDA_TRY(cudaMemset(d_dginv[1], 0, sizeof(double) * K * M));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(d_dgi, 0, sizeof(double) * std::max<size_t>(store, 1), stream));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(d_dginv[0], 0, sizeof(double) * K * M, stream));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(d_dginv[1], 0, sizeof(double) * K * M, stream));
     if ((rc = alloc_d(&d_tscal, 4 * (size_t)nmol))) return rc;
-    SFGPU_CUDA_TRY(cudaMemset(d_tscal, 0, sizeof(MolScalT) * nmol));
+    SFGPU_CUDA_TRY(cudaMemsetAsync(d_tscal, 0, sizeof(MolScalT) * nmol, stream));
     if ((rc = alloc_d(&d_dpartial, (size_t)std::max(nblocks_red, 64) * 64))) return rc;
     if ((rc = alloc_d(&d_dphib, nseg)) || (rc = alloc_d(&d_dchib, nclass))) return rc;
     if ((rc = alloc_d(&d_v, nvar)) || (rc = alloc_d(&d_jv, nvar))) return rc;
