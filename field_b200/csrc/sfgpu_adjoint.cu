@@ -357,6 +357,17 @@ void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *ds
 // 90^3 1297 / 1251, 100^3 1683 / 1770, 110^3 2039 / 2207.
 bool sfgpu_system::pair_sweeps() const { return 2 * 64.0 * M <= 100e6; }
 
+// Whether the reverse steps of a first-order lattice gather: the six-neighbour
+// and 1D/2D lattices that a grid takes, two sweeps of it in z.
+bool sfgpu_system::gathers() const {
+    const DLat &L = H.L;
+    if (K != 1 || lat_twelve(L)) return false;
+    if (L.grad < 3) return grid_fits(sites_grid(L));
+    dim3 g = cols_grid(L);
+    g.z *= 2;
+    return grid_fits(g);
+}
+
 // Gf and Gb of every position of molecule m's chain (full chains, also for
 // symmetric homopolymers) into a_gf / a_gb; with compose, the backward sweep
 // also accumulates Gf.Gb into the molecule's (zeroed) phi.  *gb0 = Gb(0).
@@ -367,7 +378,7 @@ int sfgpu_system::store_chains(int m, bool compose, const double **gb0) {
     cudaStream_t s = stream;
     const int N = o.N;
     const size_t KM = (size_t)K * M;
-    if (K == 1 && o.force == 0 && !lat_twelve(H.L) && pair_sweeps()) {
+    if (gathers() && o.force == 0 && pair_sweeps()) {
         // both recursions side by side, then the composition over the stored
         // slices: half the launches, and phi is read and written once a run
         // instead of once a step
@@ -589,7 +600,7 @@ int sfgpu_system::molecule_adjoint(int m, double *const *phibar_src) {
     const size_t KM = (size_t)K * M;
     auto GF = [&](int j) -> const double * { return (a_stride ? a_bufF : a_gf) + (size_t)j * KM; };
     auto GB = [&](int j) -> const double * { return (a_stride ? a_bufB : a_gb) + (size_t)j * KM; };
-    if (K == 1 && o.force == 0 && !lat_twelve(L)) {
+    if (gathers() && o.force == 0) {
         // gathering sweeps (adj_gather_*).  With every slice stored the two run
         // side by side, a launch taking a step of each; with checkpoints one
         // after the other, as the segments' slices pass by.

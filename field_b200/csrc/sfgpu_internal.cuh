@@ -295,6 +295,11 @@ inline dim3 sites_grid(const DLat &L) {
     return L.grad == 1 ? dim3((n + 127) / 128) : dim3((n + 31) / 32, (rows + 3) / 4);
 }
 
+// A grid is at most 65535 blocks in y and z.  A lattice whose rows or planes are
+// more than that many blocks takes the kernels that stride over a grid of fixed
+// size instead (step1_rows and its kin), as slow as they are on small lattices.
+inline bool grid_fits(dim3 g) { return g.y <= 65535u && g.z <= 65535u; }
+
 // Visit the interior sites assigned to this thread: for 1 gradient threads
 // stride over the single row; otherwise warps take rows and lanes take the
 // positions along the row.  worker = thread index among nworkers threads.

@@ -44,43 +44,41 @@ static int grid_rows(const DLat &L) {
     return (int)std::max(1L, std::min(b, 148L * 32));
 }
 
-// first-order step inside a residual evaluation: x-marching tiles on the
-// six-neighbour 3D lattices (launched as programmatic dependents of the
-// step before), row-wise otherwise
+// first-order step inside a residual evaluation, a programmatic dependent of the
+// step before: columns or x-marching tiles on the six-neighbour 3D lattices, a
+// thread per site in 1D and 2D; row-wise on the other lattices and where the
+// grid does not take the lattice (grid_fits)
 int sfgpu_system::launch_step1(const double *gin, const double *G, double *gout, const double *other, double *phi,
                                int mode) {
     const DLat &L = H.L;
-    if (L.grad == 3 && !lat_twelve(L)) {
-        const bool composing = mode != COMP_NONE;
-        const int xc = composing ? tile_xc_bwd : tile_xc;
-        dim3 grid((L.Md[2] - 2 + kTZ - 1) / kTZ, (L.Md[1] - 2 + kTY - 1) / kTY, (L.Md[0] - 2 + xc - 1) / xc);
-        const dim3 block(kTZ * kTY);
-        cudaError_t e;
-        if ((composing ? tile_pipelined_bwd : tile_pipelined) == 3) {
-            auto k = mode == COMP_ACC ? step3d_cols<COMP_ACC>
-                                      : mode == COMP_CENTRE ? step3d_cols<COMP_CENTRE> : step3d_cols<COMP_NONE>;
-            e = launch_pdl(k, cols_grid(L), dim3(32, kColY), stream, L, gin, G, gout, other, phi);
-        } else if (!composing && tile_pipelined == 2) {
-            grid.y = (L.Md[1] - 2 + kTY2 - 1) / kTY2;
-            e = launch_pdl(step3d_march_pf2, grid, block, stream, L, gin, G, gout, xc);
-        } else if (composing && tile_pipelined_bwd) {
-            e = launch_pdl(step3d_march_pf<true>, grid, block, stream, L, gin, G, gout, other, phi, mode, xc);
-        } else if (!composing && tile_pipelined) {
-            e = launch_pdl(step3d_march_pf<false>, grid, block, stream, L, gin, G, gout, other, phi, mode, xc);
-        } else {
-            e = launch_pdl(step3d_march, grid, block, stream, L, gin, G, gout, other, phi, mode, xc);
+    auto launch = [&]() -> cudaError_t {
+        if (L.grad == 3 && !lat_twelve(L)) {
+            const bool composing = mode != COMP_NONE;
+            const int form = composing ? tile_pipelined_bwd : tile_pipelined;
+            const int xc = composing ? tile_xc_bwd : tile_xc;
+            const int ty = (!composing && form == 2) ? kTY2 : kTY;
+            dim3 grid((L.Md[2] - 2 + kTZ - 1) / kTZ, (L.Md[1] - 2 + ty - 1) / ty, (L.Md[0] - 2 + xc - 1) / xc);
+            const dim3 block(kTZ * kTY);
+            if (form == 3) {
+                auto k = mode == COMP_ACC ? step3d_cols<COMP_ACC>
+                                          : mode == COMP_CENTRE ? step3d_cols<COMP_CENTRE> : step3d_cols<COMP_NONE>;
+                if (grid_fits(cols_grid(L)))
+                    return launch_pdl(k, cols_grid(L), dim3(32, kColY), stream, L, gin, G, gout, other, phi);
+            } else if (grid_fits(grid)) {
+                if (!composing && form == 2) return launch_pdl(step3d_march_pf2, grid, block, stream, L, gin, G, gout, xc);
+                if (form == 0) return launch_pdl(step3d_march, grid, block, stream, L, gin, G, gout, other, phi, mode, xc);
+                return launch_pdl(composing ? step3d_march_pf<true> : step3d_march_pf<false>, grid, block, stream, L, gin,
+                                  G, gout, other, phi, mode, xc);
+            }
+        } else if (L.grad < 3 && grid_fits(sites_grid(L))) {
+            auto k = mode == COMP_ACC ? step1_sites<COMP_ACC>
+                                      : mode == COMP_CENTRE ? step1_sites<COMP_CENTRE> : step1_sites<COMP_NONE>;
+            return launch_pdl(k, sites_grid(L), sites_block(L), stream, L, gin, G, gout, other, phi);
         }
-        if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
-    } else if (L.grad < 3) {
-        auto k = mode == COMP_ACC ? step1_sites<COMP_ACC>
-                                  : mode == COMP_CENTRE ? step1_sites<COMP_CENTRE> : step1_sites<COMP_NONE>;
-        const cudaError_t e = launch_pdl(k, sites_grid(L), sites_block(L), stream, L, gin, G, gout, other, phi);
-        if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
-    } else {
-        const cudaError_t e = launch_pdl(step1_rows, dim3(grid_rows(L)), dim3(kBlock), stream, L, gin, G, gout, other, phi,
-                                         mode);
-        if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
-    }
+        return launch_pdl(step1_rows, dim3(grid_rows(L)), dim3(kBlock), stream, L, gin, G, gout, other, phi, mode);
+    };
+    const cudaError_t e = launch();
+    if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
     return SFGPU_OK;
 }
 
@@ -90,18 +88,25 @@ int sfgpu_system::launch_step2(const double *gin, const double *G, double S, dou
     const DLat &L = H.L;
     const dim3 grid((L.Md[2] - 2 + 31) / 32, (L.Md[1] - 2 + kS2Y - 1) / kS2Y, (L.Md[0] - 2 + kS2X - 1) / kS2X);
     auto k = !backward ? step2_sites<false, false> : mode == COMP_ACC ? step2_sites<true, true> : step2_sites<true, false>;
-    const cudaError_t e = launch_pdl(k, grid, dim3(32, kS2Y, kS2X), stream, L, gin, G, S, gout, other, phi);
+    cudaError_t e;
+    if (grid_fits(grid)) {
+        e = launch_pdl(k, grid, dim3(32, kS2Y, kS2X), stream, L, gin, G, S, gout, other, phi);
+    } else {   // reads and writes the boundary copies too, which every chain's start slice holds
+        step2<<<grid_for(M), kBlock, 0, stream>>>(L, gin, G, S, gout, other, phi, mode, backward);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }
     return SFGPU_OK;
 }
 
 // lumped second-order step: step2l_sites, except at S = 0 or 1, where a weight
-// vanishes that it takes as nonzero
+// vanishes that it takes as nonzero, and where the grid does not take the lattice
 int sfgpu_system::launch_step2l(const double *gin, const double *G, double S, double *gout, const double *other,
                                 double *phi, int mode, int backward) {
     const DLat &L = H.L;
     cudaError_t e;
-    if (S == 0.0 || S == 1.0) {
+    const dim3 grid2((L.Md[1] - 2 + 31) / 32, (L.Md[0] - 2 + 3) / 4);   // 2D
+    if (S == 0.0 || S == 1.0 || (L.grad == 2 && !grid_fits(grid2))) {
         step2l_rows<<<grid_rows(L), kBlock, 0, stream>>>(L, gin, G, S, gout, other, phi, mode, backward);
         e = cudaGetLastError();
     } else if (L.grad == 1) {
@@ -109,8 +114,7 @@ int sfgpu_system::launch_step2l(const double *gin, const double *G, double S, do
         e = launch_pdl(L.cyl ? step2l_sites<3, true> : step2l_sites<3, false>, grid, dim3(128), stream, L, gin, G, S, gout,
                        other, phi, mode, backward);
     } else {
-        const dim3 grid((L.Md[1] - 2 + 31) / 32, (L.Md[0] - 2 + 3) / 4);
-        e = launch_pdl(L.cyl ? step2l_sites<5, true> : step2l_sites<5, false>, grid, dim3(32, 4), stream, L, gin, G, S,
+        e = launch_pdl(L.cyl ? step2l_sites<5, true> : step2l_sites<5, false>, grid2, dim3(32, 4), stream, L, gin, G, S,
                        gout, other, phi, mode, backward);
     }
     if (e != cudaSuccess) { sfgpu_set_error(e, "cudaLaunchKernelEx", __FILE__, __LINE__); return SFGPU_ERR_CUDA; }

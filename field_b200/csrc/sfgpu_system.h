@@ -142,6 +142,7 @@ struct sfgpu_system {
     std::vector<double *> a_phibar, a_gbar, a_phibar_raw, a_h, a_h2;
     double *a_scal = nullptr, *a_chibbar = nullptr, *a_qbar = nullptr, *a_w = nullptr, *a_xbar = nullptr;
     bool pair_sweeps() const;
+    bool gathers() const;
     int ensure_adjoint();
     int ensure_adjoint_misc();
     int store_chains(int m, bool compose, const double **gb0);

@@ -80,11 +80,11 @@ int sfgpu_system::launch_step1_t(const double *gin, const double *dgin, const do
                                  int mode) {
     const DLat &L = H.L;
     cudaError_t e;
-    if (L.grad == 3 && !lat_twelve(L)) {
+    if (L.grad == 3 && !lat_twelve(L) && grid_fits(cols_grid(L, kColsT))) {
         auto k = mode == COMP_ACC ? step3d_cols_t<COMP_ACC>
                                   : mode == COMP_CENTRE ? step3d_cols_t<COMP_CENTRE> : step3d_cols_t<COMP_NONE>;
         e = launch_pdl(k, cols_grid(L, kColsT), dim3(32, kColY), stream, L, gin, dgin, G, dG, gout, dgout, other, dother, phi, dphi);
-    } else if (L.grad < 3) {
+    } else if (L.grad < 3 && grid_fits(sites_grid(L))) {
         e = launch_pdl(step1_sites_t, sites_grid(L), sites_block(L), stream, L, gin, dgin, G, dG, gout, dgout, other,
                        dother, phi, dphi, mode);
     } else {
