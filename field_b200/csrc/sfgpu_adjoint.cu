@@ -311,14 +311,14 @@ void sfgpu_system::adj_start(const double *G, double *dst) {
     replicate<<<g, kBlock, 0, stream>>>(M, K, G, dst);
     if (K == 6) set_boundaries<<<g, kBlock, 0, stream>>>(H.L, 6, dst);
 }
-void sfgpu_system::adj_fstep(const HMol &o, int t, const double *src, double *dst) {
+int sfgpu_system::adj_fstep(const HMol &o, int t, const double *src, double *dst) {
     const DLat &L = H.L;
     const int sg = o.seg[t];
     if (K == 1 && o.force != 0)   // SF_Copol1stO.cpp:1207-1211
         step1_force_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, force_weights(L, o.force), src, d_gseg[sg], dst,
                                                                 nullptr, nullptr, COMP_NONE);
     else if (K == 1)
-        launch_step1(src, d_gseg[sg], dst, nullptr, nullptr, COMP_NONE);   // the residual's step (3D: x-marching)
+        return launch_step1(src, d_gseg[sg], dst, nullptr, nullptr, COMP_NONE);   // the residual's step
     else if (K == 6 && L.stiff) {   // SF_Copol2ndO_stiff_range.cpp:211-217, the last step isotropic
         const bool last = (t == o.N - 1);
         step2_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg],
@@ -326,11 +326,12 @@ void sfgpu_system::adj_fstep(const HMol &o, int t, const double *src, double *ds
                                                           nullptr, nullptr, COMP_NONE, 0,
                                                           last ? STEP2_ISO : STEP2_STIFF);
     } else if (K == 6)
-        launch_step2(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
+        return launch_step2(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
     else
-        launch_step2l(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
+        return launch_step2l(src, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], dst, nullptr, nullptr, COMP_NONE, 0);
+    return SFGPU_OK;
 }
-void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *dst, const double *other,
+int sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *dst, const double *other,
                              double *phi) {
     const DLat &L = H.L;
     const int sg = o.seg[t];
@@ -339,16 +340,17 @@ void sfgpu_system::adj_bstep(const HMol &o, int t, const double *src, double *ds
         step1_force_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, force_weights(L, -o.force), src, d_gseg[sg], dst,
                                                                 other, phi, mode);
     else if (K == 1)
-        launch_step1(src, d_gseg[sg], dst, other, phi, mode);
+        return launch_step1(src, d_gseg[sg], dst, other, phi, mode);
     else if (K == 6 && L.stiff) {   // :229-234, the first backward step isotropic
         const bool first = (t == o.N - 2);
         step2_rows<<<grid_rows_a(L), kBlock, 0, stream>>>(L, src, d_gseg[sg],
                                                           first ? 0.2 : pf[sg * nseg + o.seg[t + 2]], dst, other,
                                                           phi, mode, 1, first ? STEP2_ISO : STEP2_STIFF);
     } else if (K == 6)
-        launch_step2(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
+        return launch_step2(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
     else
-        launch_step2l(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
+        return launch_step2l(src, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], dst, other, phi, mode, 1);
+    return SFGPU_OK;
 }
 
 // Whether a stored chain's two sweeps run side by side: while what a reverse
@@ -415,14 +417,14 @@ int sfgpu_system::store_chains(int m, bool compose, const double **gb0) {
         return SFGPU_OK;
     }
     adj_start(d_gseg[o.seg[0]], a_gf);
-    for (int t = 1; t < N; t++) adj_fstep(o, t, a_gf + (size_t)(t - 1) * KM, a_gf + (size_t)t * KM);
+    for (int t = 1; t < N; t++) SFGPU_TRY(adj_fstep(o, t, a_gf + (size_t)(t - 1) * KM, a_gf + (size_t)t * KM));
     adj_start(d_gseg[o.seg[N - 1]], a_gb + (size_t)(N - 1) * KM);
     if (compose)
         connect<<<g, kBlock, 0, s>>>(M, K, a_gb + (size_t)(N - 1) * KM, a_gf + (size_t)(N - 1) * KM,
                                      o.d_phi[o.seg[N - 1]]);
     for (int t = N - 2; t >= 0; t--)
-        adj_bstep(o, t, a_gb + (size_t)(t + 1) * KM, a_gb + (size_t)t * KM, compose ? a_gf + (size_t)t * KM : nullptr,
-                  compose ? o.d_phi[o.seg[t]] : nullptr);
+        SFGPU_TRY(adj_bstep(o, t, a_gb + (size_t)(t + 1) * KM, a_gb + (size_t)t * KM,
+                            compose ? a_gf + (size_t)t * KM : nullptr, compose ? o.d_phi[o.seg[t]] : nullptr));
     if (gb0) *gb0 = a_gb;
     return SFGPU_OK;
 }
@@ -446,7 +448,7 @@ int sfgpu_system::store_chains_ck(int m, bool compose, const double **gb0) {
     const double *prev = a_ckF;
     for (int t = 1; t < N; t++) {
         double *dst = (t % k == 0) ? a_ckF + (size_t)(t / k) * KM : F(t & 1);
-        adj_fstep(o, t, prev, dst);
+        SFGPU_TRY(adj_fstep(o, t, prev, dst));
         prev = dst;
     }
     a_qseg = -1;
@@ -455,7 +457,7 @@ int sfgpu_system::store_chains_ck(int m, bool compose, const double **gb0) {
         const int s0 = q * k, e = std::min(s0 + k, N) - 1;
         if (compose) {   // Gf of this segment
             SFGPU_CUDA_TRY(cudaMemcpyAsync(F(0), a_ckF + (size_t)q * KM, bytes, cudaMemcpyDeviceToDevice, s));
-            for (int j = 1; j <= e - s0; j++) adj_fstep(o, s0 + j, F(j - 1), F(j));
+            for (int j = 1; j <= e - s0; j++) SFGPU_TRY(adj_fstep(o, s0 + j, F(j - 1), F(j)));
         }
         for (int t = e; t >= s0; t--) {
             double *dst = B(t - s0);
@@ -465,7 +467,7 @@ int sfgpu_system::store_chains_ck(int m, bool compose, const double **gb0) {
                 if (compose) connect<<<g, kBlock, 0, s>>>(M, K, dst, F(t - s0), o.d_phi[sg]);
             } else {
                 const double *src = (t == e) ? carry : B(t + 1 - s0);
-                adj_bstep(o, t, src, dst, compose ? F(t - s0) : nullptr, compose ? o.d_phi[sg] : nullptr);
+                SFGPU_TRY(adj_bstep(o, t, src, dst, compose ? F(t - s0) : nullptr, compose ? o.d_phi[sg] : nullptr));
             }
             if (t == e)
                 SFGPU_CUDA_TRY(cudaMemcpyAsync(a_ckB + (size_t)q * KM, dst, bytes, cudaMemcpyDeviceToDevice, s));
@@ -488,9 +490,9 @@ int sfgpu_system::load_segment(int m, int q) {
     auto F = [&](int j) { return a_bufF + (size_t)j * KM; };
     auto B = [&](int j) { return a_bufB + (size_t)j * KM; };
     SFGPU_CUDA_TRY(cudaMemcpyAsync(F(0), a_ckF + (size_t)q * KM, bytes, cudaMemcpyDeviceToDevice, s));
-    for (int j = 1; j <= e - s0; j++) adj_fstep(o, s0 + j, F(j - 1), F(j));
+    for (int j = 1; j <= e - s0; j++) SFGPU_TRY(adj_fstep(o, s0 + j, F(j - 1), F(j)));
     SFGPU_CUDA_TRY(cudaMemcpyAsync(B(e - s0), a_ckB + (size_t)q * KM, bytes, cudaMemcpyDeviceToDevice, s));
-    for (int t = e - 1; t >= s0; t--) adj_bstep(o, t, B(t + 1 - s0), B(t - s0), nullptr, nullptr);
+    for (int t = e - 1; t >= s0; t--) SFGPU_TRY(adj_bstep(o, t, B(t + 1 - s0), B(t - s0), nullptr, nullptr));
     a_qseg = q;
     return SFGPU_OK;
 }

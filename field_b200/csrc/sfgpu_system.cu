@@ -1074,9 +1074,9 @@ int sfgpu_system::molecule_phi_dend(int m) {
                     dend_combine<<<g, kBlock, 0, s>>>(M, arr, acc, Gold, ginv);
                     acc = ginv; std::swap(ginv, tmp);
                 }
-                launch_step1(acc, Gc, slice(sp), nullptr, nullptr, COMP_NONE);
+                SFGPU_TRY(launch_step1(acc, Gc, slice(sp), nullptr, nullptr, COMP_NONE));
             } else {
-                launch_step1(slice(sp - 1), Gc, slice(sp), nullptr, nullptr, COMP_NONE);
+                SFGPU_TRY(launch_step1(slice(sp - 1), Gc, slice(sp), nullptr, nullptr, COMP_NONE));
             }
             Gold = Gc;
         }
@@ -1091,7 +1091,7 @@ int sfgpu_system::molecule_phi_dend(int m) {
             const int sg = o.gen_seg[i][j - 1];
             const double *Gc = d_gseg[sg];
             if (sp == NS) SFGPU_CUDA_TRY(cudaMemcpyAsync(ginv, Gc, sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
-            else launch_step1(cur, Gc, ginv, nullptr, nullptr, COMP_NONE);
+            else SFGPU_TRY(launch_step1(cur, Gc, ginv, nullptr, nullptr, COMP_NONE));
             cur = ginv; std::swap(ginv, tmp);
             if (j == 1)
                 for (int k = 1; k <= rep - 1; k++) {
@@ -1205,7 +1205,7 @@ int sfgpu_system::molecule_phi_tree(int m) {
                 w ^= 1;
             }
         }
-        if (q > 0) launch_step1(U(q), d_gseg[o.seg[o.parent[q]]], Q(q), nullptr, nullptr, COMP_NONE);
+        if (q > 0) SFGPU_TRY(launch_step1(U(q), d_gseg[o.seg[o.parent[q]]], Q(q), nullptr, nullptr, COMP_NONE));
     }
     // from segment 0 outwards, composing every segment
     SFGPU_CUDA_TRY(cudaMemcpyAsync(D(0), d_gseg[o.seg[0]], bytes, cudaMemcpyDeviceToDevice, s));
@@ -1223,7 +1223,7 @@ int sfgpu_system::molecule_phi_tree(int m) {
                 acc = tmp[w];
                 w ^= 1;
             }
-            launch_step1(acc, d_gseg[o.seg[c]], D(c), nullptr, nullptr, COMP_NONE);
+            SFGPU_TRY(launch_step1(acc, d_gseg[o.seg[c]], D(c), nullptr, nullptr, COMP_NONE));
         }
     }
     MolParam p;
@@ -1293,15 +1293,15 @@ int sfgpu_system::molecule_phi(int m) {
         double *phi = o.d_phi[i];
         SFGPU_CUDA_TRY(cudaMemcpyAsync(d_gi, G, sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         for (int t = 1; t < half; t++)
-            launch_step1(d_gi + (size_t)(t - 1) * M, G, d_gi + (size_t)t * M, nullptr, nullptr, COMP_NONE);
+            SFGPU_TRY(launch_step1(d_gi + (size_t)(t - 1) * M, G, d_gi + (size_t)t * M, nullptr, nullptr, COMP_NONE));
         const double *cur = d_gi + (size_t)(half - 1) * M;
         if (N % 2 == 1) {
-            launch_step1(cur, G, ginv, nullptr, phi, COMP_CENTRE);
+            SFGPU_TRY(launch_step1(cur, G, ginv, nullptr, phi, COMP_CENTRE));
             cur = ginv; std::swap(ginv, tmp);
         }
         for (int sp = (N + 3) / 2; sp <= N; sp++) {
             int sinv = N - sp + 1;
-            launch_step1(cur, G, ginv, d_gi + (size_t)(sinv - 1) * M, phi, COMP_ACC);
+            SFGPU_TRY(launch_step1(cur, G, ginv, d_gi + (size_t)(sinv - 1) * M, phi, COMP_ACC));
             cur = ginv; std::swap(ginv, tmp);
         }
         wsum_partial<<<nblocks_red, kBlock, 0, s>>>(M, 1, cur, d_wgn, d_partial);
@@ -1313,45 +1313,48 @@ int sfgpu_system::molecule_phi(int m) {
     // full storage: copolymers and all second-order chains
     const int N = o.N;
     // forward step into position t (SF_Copol1stO::Matrix1 / SF_Copol2ndO::Matrix1)
-    auto fwd = [&](int t, const double *in, double *out) {
+    auto fwd = [&](int t, const double *in, double *out) -> int {
         int sg = o.seg[t];
         if (K == 1 && o.force != 0)   // SF_Copol1stO.cpp:1207-1211: PropagateG(Gi, G, s, force)
             step1_force_rows<<<grid_rows(L), kBlock, 0, s>>>(L, force_weights(L, o.force), in, d_gseg[sg], out,
                                                              nullptr, nullptr, COMP_NONE);
         else if (K == 1)
-            launch_step1(in, d_gseg[sg], out, nullptr, nullptr, COMP_NONE);
+            return launch_step1(in, d_gseg[sg], out, nullptr, nullptr, COMP_NONE);
         else if (K == 6 && L.stiff) {
             // SF_Copol2ndO_stiff_range::Matrix1 (SF_Copol2ndO_stiff_range.cpp:211-217):
             // step s (1-based) takes Pf(s-1, s+1); the last one is isotropic
             const bool last = (t == N - 1);
             const double Sv = last ? 0.2 : pf[o.seg[t - 1] * nseg + o.seg[t + 1]];
-            launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg], Sv, out,
-                       (const double *)nullptr, (double *)nullptr, (int)COMP_NONE, 0,
-                       (int)(last ? STEP2_ISO : STEP2_STIFF));
+            SFGPU_CUDA_TRY(launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg],
+                                      Sv, out, (const double *)nullptr, (double *)nullptr, (int)COMP_NONE, 0,
+                                      (int)(last ? STEP2_ISO : STEP2_STIFF)));
         } else if (K == 6)
-            launch_step2(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
+            return launch_step2(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
         else
-            launch_step2l(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
+            return launch_step2l(in, d_gseg[sg], pf[o.seg[t - 1] * nseg + sg], out, nullptr, nullptr, COMP_NONE, 0);
+        return SFGPU_OK;
     };
     // backward step into position t with the composition phi += Gb(t) Gf(t)
-    auto bwd = [&](int t, const double *in, double *out, const double *gf) {
+    auto bwd = [&](int t, const double *in, double *out, const double *gf) -> int {
         int sg = o.seg[t];
         if (K == 1 && o.force != 0)   // backward steps with -force (SF_Copol1stO.cpp:1226-1230)
             step1_force_rows<<<grid_rows(L), kBlock, 0, s>>>(L, force_weights(L, -o.force), in, d_gseg[sg], out, gf,
                                                              o.d_phi[sg], COMP_ACC);
         else if (K == 1)
-            launch_step1(in, d_gseg[sg], out, gf, o.d_phi[sg], COMP_ACC);
+            return launch_step1(in, d_gseg[sg], out, gf, o.d_phi[sg], COMP_ACC);
         else if (K == 6 && L.stiff) {
             // backward step s (1-based) takes Pf(s, s+2); the first one
             // (s = N-1) is isotropic (SF_Copol2ndO_stiff_range.cpp:229-234)
             const bool first = (t == N - 2);
             const double Sv = first ? 0.2 : pf[sg * nseg + o.seg[t + 2]];
-            launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg], Sv, out, gf,
-                       o.d_phi[sg], (int)COMP_ACC, 1, (int)(first ? STEP2_ISO : STEP2_STIFF));
+            SFGPU_CUDA_TRY(launch_pdl(step2_rows, dim3(grid_rows(L)), dim3(kBlock), s, L, in, (const double *)d_gseg[sg],
+                                      Sv, out, gf, o.d_phi[sg], (int)COMP_ACC, 1,
+                                      (int)(first ? STEP2_ISO : STEP2_STIFF)));
         } else if (K == 6)
-            launch_step2(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
+            return launch_step2(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
         else
-            launch_step2l(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
+            return launch_step2l(in, d_gseg[sg], pf[sg * nseg + o.seg[t + 1]], out, gf, o.d_phi[sg], COMP_ACC, 1);
+        return SFGPU_OK;
     };
     const bool ori = orient && K > 1;
     // storage: every slice, or checkpoints ck[q] = Gf(qk) plus one segment
@@ -1367,7 +1370,7 @@ int sfgpu_system::molecule_phi(int m) {
     };
     replicate<<<g, kBlock, 0, s>>>(M, K, d_gseg[o.seg[0]], slot(0));
     if (K == 6) set_boundaries<<<g, kBlock, 0, s>>>(L, 6, slot(0));
-    for (int t = 1; t < N; t++) fwd(t, slot(t - 1), slot(t));
+    for (int t = 1; t < N; t++) SFGPU_TRY(fwd(t, slot(t - 1), slot(t)));
     replicate<<<g, kBlock, 0, s>>>(M, K, d_gseg[o.seg[N - 1]], ginv);
     if (K == 6) set_boundaries<<<g, kBlock, 0, s>>>(L, 6, ginv);
     connect<<<g, kBlock, 0, s>>>(M, K, ginv, slot(N - 1), o.d_phi[o.seg[N - 1]]);
@@ -1381,10 +1384,10 @@ int sfgpu_system::molecule_phi(int m) {
     for (int t = N - 2; t >= 0; t--) {
         if (ckpt && t % kst != 0 && t / kst != seg_held) {
             const int q = t / kst;   // recompute Gf(qk+1 .. qk+k-1) from ck[q]
-            for (int u = q * kst + 1; u <= std::min(q * kst + kst - 1, N - 1); u++) fwd(u, slot(u - 1), slot(u));
+            for (int u = q * kst + 1; u <= std::min(q * kst + kst - 1, N - 1); u++) SFGPU_TRY(fwd(u, slot(u - 1), slot(u)));
             seg_held = q;
         }
-        bwd(t, cur, ginv, slot(t));
+        SFGPU_TRY(bwd(t, cur, ginv, slot(t)));
         if (ori) orient_acc<<<g, kBlock, 0, s>>>(L, ginv, slot(t), o.d_ori[o.seg[t]]);
         cur = ginv; std::swap(ginv, tmp);
     }
@@ -2027,35 +2030,31 @@ extern "C" int sfgpu_profile_propagator(sfgpu_system *s, int reps, double *ms_fw
     if (nslices < 2) return fail(SFGPU_ERR_INVALID, "chain too short to time");
     const double *G = s->d_gseg[o.seg[0]];
     double *phi = o.d_phi[o.seg[0]];
-    const int g = grid_for(M);
-    cudaEvent_t e0, e1, e2;
-    SFGPU_CUDA_TRY(cudaEventCreate(&e0));
-    SFGPU_CUDA_TRY(cudaEventCreate(&e1));
-    SFGPU_CUDA_TRY(cudaEventCreate(&e2));
-    SFGPU_CUDA_TRY(cudaEventRecord(e0, s->stream));
+    auto step = [&](const double *in, double *out, const double *other, double *acc, int mode, int backward) -> int {
+        if (K == 1) return s->launch_step1(in, G, out, other, acc, mode);
+        if (K == 6) return s->launch_step2(in, G, 0.2, out, other, acc, mode, backward);
+        return s->launch_step2l(in, G, 0.2, out, other, acc, mode, backward);
+    };
+    struct Events {
+        cudaEvent_t e[3] = {};
+        ~Events() { for (cudaEvent_t v : e) if (v) cudaEventDestroy(v); }
+    } ev;
+    for (cudaEvent_t &v : ev.e) SFGPU_CUDA_TRY(cudaEventCreate(&v));
+    SFGPU_CUDA_TRY(cudaEventRecord(ev.e[0], s->stream));
     for (int r = 0; r < reps; r++) {
         size_t t = 1 + (size_t)r % (nslices - 1);
-        if (K == 1)
-            s->launch_step1(s->d_gi + (t - 1) * KM, G, s->d_gi + t * KM, nullptr, nullptr, COMP_NONE);
-        else
-            s->launch_step2(s->d_gi + (t - 1) * KM, G, 0.2, s->d_gi + t * KM, nullptr, nullptr, COMP_NONE, 0);
+        SFGPU_TRY(step(s->d_gi + (t - 1) * KM, s->d_gi + t * KM, nullptr, nullptr, COMP_NONE, 0));
     }
-    SFGPU_CUDA_TRY(cudaEventRecord(e1, s->stream));
+    SFGPU_CUDA_TRY(cudaEventRecord(ev.e[1], s->stream));
     for (int r = 0; r < reps; r++) {
         size_t t = (size_t)r % nslices;
-        const double *src = s->d_ginv[r & 1];
-        double *dst = s->d_ginv[(r + 1) & 1];
-        if (K == 1)
-            s->launch_step1(src, G, dst, s->d_gi + t * KM, phi, COMP_ACC);
-        else
-            s->launch_step2(src, G, 0.2, dst, s->d_gi + t * KM, phi, COMP_ACC, 1);
+        SFGPU_TRY(step(s->d_ginv[r & 1], s->d_ginv[(r + 1) & 1], s->d_gi + t * KM, phi, COMP_ACC, 1));
     }
-    SFGPU_CUDA_TRY(cudaEventRecord(e2, s->stream));
-    SFGPU_CUDA_TRY(cudaEventSynchronize(e2));
+    SFGPU_CUDA_TRY(cudaEventRecord(ev.e[2], s->stream));
+    SFGPU_CUDA_TRY(cudaEventSynchronize(ev.e[2]));
     float a = 0, b = 0;
-    SFGPU_CUDA_TRY(cudaEventElapsedTime(&a, e0, e1));
-    SFGPU_CUDA_TRY(cudaEventElapsedTime(&b, e1, e2));
-    cudaEventDestroy(e0); cudaEventDestroy(e1); cudaEventDestroy(e2);
+    SFGPU_CUDA_TRY(cudaEventElapsedTime(&a, ev.e[0], ev.e[1]));
+    SFGPU_CUDA_TRY(cudaEventElapsedTime(&b, ev.e[1], ev.e[2]));
     if (ms_fwd) *ms_fwd = a / reps;
     if (ms_bwd) *ms_bwd = b / reps;
     if (bytes_fwd) *bytes_fwd = 8.0 * (2 * K + 1) * M;

@@ -27,6 +27,13 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
 // when the call returns, a clear always).
 int sfgpu_after_setup(cudaStream_t stream);
 
+// returns a status that is not SFGPU_OK from the enclosing function
+#define SFGPU_TRY(call)                    \
+    do {                                   \
+        const int rc_try = (call);         \
+        if (rc_try) return rc_try;         \
+    } while (0)
+
 struct GroupShape;
 namespace sfb { struct InstDesc; }
 
@@ -149,8 +156,8 @@ struct sfgpu_system {
     int store_chains_ck(int m, bool compose, const double **gb0);
     int load_segment(int m, int q);
     void adj_start(const double *G, double *dst);
-    void adj_fstep(const HMol &o, int t, const double *src, double *dst);
-    void adj_bstep(const HMol &o, int t, const double *src, double *dst, const double *other, double *phi);
+    int adj_fstep(const HMol &o, int t, const double *src, double *dst);
+    int adj_bstep(const HMol &o, int t, const double *src, double *dst, const double *other, double *phi);
     int set_checkpoint(int stride);
     int molecule_phi_store(int m);
     int molecule_adjoint(int m, double *const *phibar_src);

@@ -160,8 +160,8 @@ int sfgpu_system::molecule_phi_t(int m) {
             SFGPU_CUDA_TRY(cudaMemsetAsync(o.d_dphi[i], 0, bytes, s));
         }
         auto stepT = [&](const double *in, const double *din, int sgq, double *out, double *dout) {
-            launch_step1_t(in, din, d_gseg[sgq], dgseg[sgq], out, dout, nullptr, nullptr,
-                           nullptr, nullptr, COMP_NONE);
+            return launch_step1_t(in, din, d_gseg[sgq], dgseg[sgq], out, dout, nullptr, nullptr, nullptr, nullptr,
+                                  COMP_NONE);
         };
         for (int q = N - 1; q >= 0; q--) {
             const int sq = o.seg[q];
@@ -184,7 +184,7 @@ int sfgpu_system::molecule_phi_t(int m) {
                     w ^= 1;
                 }
             }
-            if (q > 0) stepT(U(q), dU(q), o.seg[o.parent[q]], Q(q), dQ(q));
+            if (q > 0) SFGPU_TRY(stepT(U(q), dU(q), o.seg[o.parent[q]], Q(q), dQ(q)));
         }
         SFGPU_CUDA_TRY(cudaMemcpyAsync(D(0), d_gseg[o.seg[0]], bytes, cudaMemcpyDeviceToDevice, s));
         SFGPU_CUDA_TRY(cudaMemcpyAsync(dD(0), dgseg[o.seg[0]], bytes, cudaMemcpyDeviceToDevice, s));
@@ -202,7 +202,7 @@ int sfgpu_system::molecule_phi_t(int m) {
                     acc = d_ginv[w]; dacc = d_dginv[w];
                     w ^= 1;
                 }
-                stepT(acc, dacc, o.seg[c], D(c), dD(c));
+                SFGPU_TRY(stepT(acc, dacc, o.seg[c], D(c), dD(c)));
             }
         }
         cur = U(0);
@@ -221,20 +221,20 @@ int sfgpu_system::molecule_phi_t(int m) {
         SFGPU_CUDA_TRY(cudaMemcpyAsync(t_gi, G, sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         SFGPU_CUDA_TRY(cudaMemcpyAsync(d_dgi, dG, sizeof(double) * M, cudaMemcpyDeviceToDevice, s));
         for (int t = 1; t < half; t++)
-            launch_step1_t(t_gi + (size_t)(t - 1) * M, d_dgi + (size_t)(t - 1) * M, G, dG,
-                           t_gi + (size_t)t * M, d_dgi + (size_t)t * M, nullptr, nullptr,
-                           nullptr, nullptr, COMP_NONE);
+            SFGPU_TRY(launch_step1_t(t_gi + (size_t)(t - 1) * M, d_dgi + (size_t)(t - 1) * M, G, dG,
+                                     t_gi + (size_t)t * M, d_dgi + (size_t)t * M, nullptr, nullptr, nullptr, nullptr,
+                                     COMP_NONE));
         cur = t_gi + (size_t)(half - 1) * M;
         dcur = d_dgi + (size_t)(half - 1) * M;
         if (N % 2 == 1) {
-            launch_step1_t(cur, dcur, G, dG, ginv, dginv, nullptr, nullptr, phi, dph, COMP_CENTRE);
+            SFGPU_TRY(launch_step1_t(cur, dcur, G, dG, ginv, dginv, nullptr, nullptr, phi, dph, COMP_CENTRE));
             cur = ginv; dcur = dginv;
             std::swap(ginv, tmp); std::swap(dginv, dtmp);
         }
         for (int sp = (N + 3) / 2; sp <= N; sp++) {
             int sinv = N - sp + 1;
-            launch_step1_t(cur, dcur, G, dG, ginv, dginv, t_gi + (size_t)(sinv - 1) * M,
-                           d_dgi + (size_t)(sinv - 1) * M, phi, dph, COMP_ACC);
+            SFGPU_TRY(launch_step1_t(cur, dcur, G, dG, ginv, dginv, t_gi + (size_t)(sinv - 1) * M,
+                                     d_dgi + (size_t)(sinv - 1) * M, phi, dph, COMP_ACC));
             cur = ginv; dcur = dginv;
             std::swap(ginv, tmp); std::swap(dginv, dtmp);
         }
@@ -246,7 +246,7 @@ int sfgpu_system::molecule_phi_t(int m) {
         // (molecule_phi: SF_Copol2ndO_stiff_range.cpp:211-234 for the stiff
         // range's Pf(s-1, s+1) and isotropic end steps)
         const bool pair = (K == 3 || K == 5) || (K == 6 && L.stiff);
-        auto prim = [&](int t, bool backward, const double *in, const double *G, double *out) {
+        auto prim = [&](int t, bool backward, const double *in, const double *G, double *out) -> int {
             const int sg = o.seg[t];
             if (K == 6) {
                 const bool iso = backward ? (t == N - 2) : (t == N - 1);
@@ -255,15 +255,17 @@ int sfgpu_system::molecule_phi_t(int m) {
                                                  iso ? STEP2_ISO : STEP2_STIFF);
             } else {
                 const double Sv = backward ? pf[sg * nseg + o.seg[t + 1]] : pf[o.seg[t - 1] * nseg + sg];
-                launch_step2l(in, G, Sv, out, nullptr, nullptr, COMP_NONE, backward ? 1 : 0);
+                return launch_step2l(in, G, Sv, out, nullptr, nullptr, COMP_NONE, backward ? 1 : 0);
             }
+            return SFGPU_OK;
         };
-        auto pair_step = [&](int t, bool backward, const double *in, const double *din, double *out, double *dout) {
+        auto pair_step = [&](int t, bool backward, const double *in, const double *din, double *out, double *dout) -> int {
             const int sg = o.seg[t];
-            prim(t, backward, in, d_gseg[sg], out);
-            prim(t, backward, din, d_gseg[sg], t_w[0]);
-            prim(t, backward, in, dgseg[sg], t_w[1]);
+            SFGPU_TRY(prim(t, backward, in, d_gseg[sg], out));
+            SFGPU_TRY(prim(t, backward, din, d_gseg[sg], t_w[0]));
+            SFGPU_TRY(prim(t, backward, in, dgseg[sg], t_w[1]));
             sum2<<<g, kBlock, 0, s>>>(KM, t_w[0], t_w[1], dout);
+            return SFGPU_OK;
         };
         replicate<<<g, kBlock, 0, s>>>(M, K, d_gseg[o.seg[0]], t_gi);
         replicate<<<g, kBlock, 0, s>>>(M, K, dgseg[o.seg[0]], d_dgi);
@@ -272,13 +274,13 @@ int sfgpu_system::molecule_phi_t(int m) {
             const double *src = t_gi + (size_t)(t - 1) * KM, *dsrc = d_dgi + (size_t)(t - 1) * KM;
             double *dst = t_gi + (size_t)t * KM, *ddst = d_dgi + (size_t)t * KM;
             if (pair)
-                pair_step(t, false, src, dsrc, dst, ddst);
+                SFGPU_TRY(pair_step(t, false, src, dsrc, dst, ddst));
             else if (K == 1 && o.force != 0)   // forward steps with +force
                 step1_force_rows_t<<<gr, kBlock, 0, s>>>(L, force_weights(L, o.force), src, dsrc, d_gseg[sg], dgseg[sg],
                                                          dst, ddst, nullptr, nullptr, nullptr, nullptr, COMP_NONE);
             else if (K == 1)
-                launch_step1_t(src, dsrc, d_gseg[sg], dgseg[sg], dst, ddst, nullptr, nullptr,
-                           nullptr, nullptr, COMP_NONE);
+                SFGPU_TRY(launch_step1_t(src, dsrc, d_gseg[sg], dgseg[sg], dst, ddst, nullptr, nullptr, nullptr, nullptr,
+                                         COMP_NONE));
             else
                 step2_rows_t<<<gr, kBlock, 0, s>>>(L, src, dsrc, d_gseg[sg], dgseg[sg], pf[o.seg[t - 1] * nseg + sg],
                                                    dst, ddst, nullptr, nullptr, nullptr, nullptr, COMP_NONE, 0);
@@ -292,7 +294,7 @@ int sfgpu_system::molecule_phi_t(int m) {
         for (int t = N - 2; t >= 0; t--) {
             int sg = o.seg[t];
             if (pair) {
-                pair_step(t, true, cur, dcur, ginv, dginv);
+                SFGPU_TRY(pair_step(t, true, cur, dcur, ginv, dginv));
                 compose2_t<<<g, kBlock, 0, s>>>(L, K, ginv, dginv, t_gi + (size_t)t * KM, d_dgi + (size_t)t * KM,
                                                 o.d_phi[sg], o.d_dphi[sg]);
             } else if (K == 1 && o.force != 0)   // backward steps with -force
@@ -300,9 +302,8 @@ int sfgpu_system::molecule_phi_t(int m) {
                                                          dgseg[sg], ginv, dginv, t_gi + (size_t)t * KM,
                                                          d_dgi + (size_t)t * KM, o.d_phi[sg], o.d_dphi[sg], COMP_ACC);
             else if (K == 1)
-                launch_step1_t(cur, dcur, d_gseg[sg], dgseg[sg], ginv, dginv,
-                           t_gi + (size_t)t * KM, d_dgi + (size_t)t * KM, o.d_phi[sg],
-                           o.d_dphi[sg], COMP_ACC);
+                SFGPU_TRY(launch_step1_t(cur, dcur, d_gseg[sg], dgseg[sg], ginv, dginv, t_gi + (size_t)t * KM,
+                                         d_dgi + (size_t)t * KM, o.d_phi[sg], o.d_dphi[sg], COMP_ACC));
             else
                 step2_rows_t<<<gr, kBlock, 0, s>>>(L, cur, dcur, d_gseg[sg], dgseg[sg], pf[sg * nseg + o.seg[t + 1]],
                                                    ginv, dginv, t_gi + (size_t)t * KM, d_dgi + (size_t)t * KM,
