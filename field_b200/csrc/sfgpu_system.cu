@@ -654,6 +654,7 @@ int sfgpu_system::setup(const sfgpu_system_desc *d) {
         store = std::max(store, need);
     }
     if ((rc = alloc_d(&d_gi, store))) return rc;
+    gi_doubles = store;
     if ((rc = alloc_d(&d_ginv[0], (size_t)K * M)) || (rc = alloc_d(&d_ginv[1], (size_t)K * M))) return rc;
     // row-wise steps never write boundary entries; surface layers are read
     // in place and must hold the propagator's value there, 0
@@ -2026,7 +2027,9 @@ extern "C" int sfgpu_profile_propagator(sfgpu_system *s, int reps, double *ms_fw
     const HMol &o = s->mols[mol];
     const int K = s->K, M = s->M;
     const size_t KM = (size_t)K * M;
-    size_t nslices = (size_t)(o.sym ? std::max(1, o.N / 2) : o.N);
+    // no more slices than are stored: a checkpointed chain or a dendrimer keeps
+    // fewer than its length
+    const size_t nslices = std::min((size_t)(o.sym ? std::max(1, o.N / 2) : o.N), s->gi_doubles / KM);
     if (nslices < 2) return fail(SFGPU_ERR_INVALID, "chain too short to time");
     const double *G = s->d_gseg[o.seg[0]];
     double *phi = o.d_phi[o.seg[0]];

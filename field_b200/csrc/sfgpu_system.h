@@ -91,6 +91,7 @@ struct sfgpu_system {
     int *d_jmap = nullptr, *d_sites = nullptr;
     std::vector<double *> d_range, d_gfull, d_gseg, d_phi;
     double *d_gi = nullptr, *d_ginv[2] = {nullptr, nullptr};
+    size_t gi_doubles = 0;
     double *d_partial = nullptr, *d_scal = nullptr, *d_phib = nullptr, *d_chib = nullptr, *d_misc = nullptr;
     double *d_x = nullptr, *d_f = nullptr;
     int nblocks_red = 1;

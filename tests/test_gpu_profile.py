@@ -33,3 +33,14 @@ def test_profile_times_every_lattice(n, order, geometry):
     # a launch takes microseconds at least; forty that never ran take less than that together
     assert p["ms_fwd"] > 5e-4 and p["ms_bwd"] > 5e-4
     assert np.array_equal(s.residual(x), f)
+
+
+@pytest.mark.parametrize("n,order", [((20, 33), 1), ((9, 8, 33), 1), ((9, 8, 33), 2)])
+def test_profile_of_a_checkpointed_chain(n, order):
+    """Of 17 slices a stride of 5 keeps 4 checkpoints and 5: the profile stays within them."""
+    s = system(n, order, checkpoint_stride=5)
+    x = np.random.default_rng(1).normal(0, 0.2, s.nvar)
+    f = s.residual(x)
+    s.profile_propagator(reps=40)
+    s.autotune(reps=3)
+    assert np.array_equal(s.residual(x), f)
