@@ -105,7 +105,7 @@ static void configure_group(sfgpu_batch *b) {
     long sites = 1;
     for (auto *s : b->sys) {
         const DLat &L = s->H.L;
-        if (!s->group || L.grad != s0->H.L.grad || (L.cyl != 0) != (s0->H.L.cyl != 0)) return;
+        if (!group_eligible(s) || L.grad != s0->H.L.grad || (L.cyl != 0) != (s0->H.L.cyl != 0)) return;
         if (L.grad == 2) sites = std::max(sites, (long)(L.Md[0] - 2) * (L.Md[1] - 2));
     }
     int C = 1, threads = 256;
@@ -139,6 +139,46 @@ static void configure_group(sfgpu_batch *b) {
     b->grouped = true;
 }
 
+// Tables and working memory of all instances, in one allocation each and one copy
+// (256 uneven 1D systems of up to 400 layers and 1000 segments: 78 ms to create
+// and 116 MiB; with allocations and copies per instance, and slices beside d_gi,
+// 112 ms and 176 MiB).  chains[i]: instance i's chain tables.
+static int upload_tables(sfgpu_batch *b, std::vector<const int *> *chains) {
+    const size_t n = b->sys.size();
+    std::vector<int> tables;
+    std::vector<size_t> maps(n), at(n), part(n), slices(n);
+    size_t doubles = 0;
+    auto take = [&](size_t k) { const size_t r = doubles; doubles += (k + 1) / 2 * 2; return r; };   // 16-byte aligned
+    for (size_t i = 0; i < n; i++) {
+        sfgpu_system *s = b->sys[i];
+        maps[i] = tables.size();
+        if (b->grouped) {
+            s->site_maps(&tables);
+            part[i] = take((size_t)s->nmol * ((s->M + 255) / 256));
+            slices[i] = take(group_slices(s, b->shape));
+        }
+        std::vector<int>().swap(s->jmap_h);
+        at[i] = tables.size();
+        s->chain_tables(&tables);
+    }
+    int *d = nullptr, rc;
+    double *w = nullptr;
+    if ((rc = balloc(b, (void **)&d, sizeof(int) * tables.size()))) return rc;
+    if (b->grouped && (rc = balloc(b, (void **)&w, sizeof(double) * doubles))) return rc;
+    SFGPU_CUDA_TRY(cudaMemcpy(d, tables.data(), sizeof(int) * tables.size(), cudaMemcpyHostToDevice));
+    for (size_t i = 0; i < n; i++) {
+        sfgpu_system *s = b->sys[i];
+        (*chains)[i] = d + at[i];
+        if (!b->grouped) continue;
+        s->d_smap = d + maps[i];
+        s->d_jall = s->d_smap + s->M;
+        s->d_wpart = w + part[i];
+        s->d_slices1 = w + slices[i];
+        if ((rc = s->clear_profiles())) return rc;
+    }
+    return SFGPU_OK;
+}
+
 extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, sfgpu_batch **out) {
     if (!out || !descs || n < 1) return SFGPU_ERR_INVALID;
     *out = nullptr;
@@ -168,8 +208,7 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
         if (descs[i].lattice.gradients == 3 && descs[i].lattice.lattice_type != SFGPU_LATTICE_STANDARD) b->wide = true;
         sfgpu_system *s = new sfgpu_system();
         s->stream = b->stream;
-        rc = s->setup(&descs[i]);
-        if (!rc) rc = s->setup_group();
+        rc = s->setup(&descs[i], false);
         if (!rc && (s->nseg > kResMax || s->nclass > kResMax)) rc = SFGPU_ERR_UNSUPPORTED;   // site_residual registers
         if (rc) { delete s; break; }
         b->sys.push_back(s);
@@ -178,6 +217,14 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
         maxM = std::max(maxM, s->M);
     }
     if (rc) { delete b; return rc; }
+    configure_group(b);
+    // chain storage: the engine keeps a 1D chain in slices of its own, everything
+    // else in d_gi
+    for (auto *s : b->sys)
+        if (!rc && !(b->grouped && s->H.L.grad == 1)) rc = s->alloc_chains();
+    std::vector<const int *> chains(n);
+    if (!rc) rc = upload_tables(b, &chains);
+    if (rc) { delete b; return rc; }
     // concatenated iteration variables and per-instance DIIS work
     if ((rc = balloc(b, (void **)&b->d_xall, sizeof(double) * b->total))) { delete b; return rc; }
     b->desc_h.resize(n);
@@ -185,8 +232,7 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
         sfgpu_system *s = b->sys[i];
         InstDesc &I = b->desc_h[i];
         fill_inst_desc(s, &I);
-        rc = s->upload_chains(&I);
-        if (rc) break;
+        s->point_chains(chains[i], &I);
         {   // force ensembles: step weights per molecule
             std::vector<sfk::ForceW> fw(2 * s->nmol);
             I.fmask = 0;
@@ -222,7 +268,6 @@ extern "C" int sfgpu_batch_create(int n, const sfgpu_system_desc *descs, int m, 
     // on the uneven 1D sweep, where 384 beat 256 by 4.5 % and 32..128 lost)
     b->block = maxM >= 4096 ? 1024 : (maxM >= 1024 ? 512 : (maxM >= 384 ? 384 : 256));
     if ((rc = configure_stage(b, true))) { delete b; return rc; }
-    configure_group(b);
     if ((rc = sfgpu_after_setup(b->stream))) { delete b; return rc; }
     *out = b;
     return SFGPU_OK;

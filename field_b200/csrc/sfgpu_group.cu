@@ -267,6 +267,32 @@ bool group_eligible(const sfgpu_system *s) {
     return true;
 }
 
+// what a 1D system asks of shared memory: exchange lines and the ring, its
+// working arrays, and the stored slices of its longest chain
+struct Doubles1 { size_t always, arrays, chain; };
+static Doubles1 doubles1(const sfgpu_system *s) {
+    const int n = s->H.L.Md[0] - 2;
+    int nonfrozen = 0, pinned = 0, molphis = 0;
+    Doubles1 q = {line1d(n) + kRing1 * slice1d(n), 0, 0};
+    for (int i = 0; i < s->nseg; i++) {
+        nonfrozen += s->freedom[i] != SFGPU_SEG_FROZEN;
+        pinned += s->freedom[i] == SFGPU_SEG_PINNED;
+    }
+    for (const auto &o : s->mols) {
+        molphis += (int)o.used.size();
+        if (o.type != 0) q.chain = std::max(q.chain, (size_t)(o.sym ? o.N / 2 : o.N) * slice1d(n));
+    }
+    q.arrays = local1d_doubles(s->M, s->nseg, nonfrozen, pinned, molphis, s->nmol);
+    return q;
+}
+
+// as localize1d decides it
+size_t group_slices(const sfgpu_system *s, const GroupShape &g) {
+    if (g.dim != 1) return 0;
+    const Doubles1 q = doubles1(s);
+    return q.always + q.arrays + q.chain <= g.smem / sizeof(double) ? 0 : q.chain;
+}
+
 // Blocks per cluster, rows per thread and threads of one system when `blocks`
 // blocks at most work on it.  Rows per thread: the fewest whose threads stay
 // within `threads`, so that a block's steps have many warps to hide their
@@ -286,22 +312,12 @@ bool group_shape(const sfgpu_system *s, int blocks, int threads, int m, GroupSha
         // share an SM in a large batch, whose registers then hold 128 each
         g.threads = std::max(blocks > 1 ? 256 : 128, 32 * warps1d(n));
         // what localize1d takes, in its order; the last ones only where they fit
-        size_t chain = 0;
-        int nonfrozen = 0, pinned = 0, molphis = 0;
-        for (int i = 0; i < s->nseg; i++) {
-            nonfrozen += s->freedom[i] != SFGPU_SEG_FROZEN;
-            pinned += s->freedom[i] == SFGPU_SEG_PINNED;
-        }
-        for (const auto &o : s->mols) {
-            molphis += (int)o.used.size();
-            if (o.type != 0) chain = std::max(chain, (size_t)(o.sym ? o.N / 2 : o.N) * slice1d(n));
-        }
-        size_t d = line1d(n) + kRing1 * slice1d(n);
+        const Doubles1 need = doubles1(s);
+        size_t d = need.always;
         const size_t most = kSmemMax / sizeof(double) / (blocks > 1 ? 1 : 2);
-        const size_t arrays = local1d_doubles(s->M, s->nseg, nonfrozen, pinned, molphis, s->nmol);
-        if (d + arrays <= most) {
-            d += arrays;
-            if (d + chain <= most) d += chain;
+        if (d + need.arrays <= most) {
+            d += need.arrays;
+            if (d + need.chain <= most) d += need.chain;
             const size_t nv = s->nvar;
             if (m > 0 && d + 2 * nv <= most) {
                 d += 2 * nv;

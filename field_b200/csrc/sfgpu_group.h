@@ -26,6 +26,9 @@ bool group_eligible(const sfgpu_system *s);
 // slices fill shared memory); threads: most threads a 2D block should take
 // m: Pure_DIIS's memory, 0 for a residual evaluation
 bool group_shape(const sfgpu_system *s, int blocks, int threads, int m, GroupShape *out);
+// doubles of stored slices that a 1D system keeps in global memory under the
+// shape: 0 where its chains fit into shared memory
+size_t group_slices(const sfgpu_system *s, const GroupShape &shape);
 int group_prepare(const GroupShape &s, bool diis);
 int group_max_clusters(const GroupShape &s, bool diis);
 int group_residual(const GroupShape &s, const sfb::InstDesc *desc, const double *x, double *f, cudaStream_t st);

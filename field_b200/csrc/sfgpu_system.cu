@@ -369,7 +369,7 @@ int sfgpu_system::alloc_i(int **p, size_t n) {
     return rc;
 }
 
-int sfgpu_system::setup(const sfgpu_system_desc *d) {
+int sfgpu_system::setup(const sfgpu_system_desc *d, bool chains) {
     int rc = sfgpu_build_lattice(&d->lattice, &H);
     if (rc) return rc;
     DLat &L = H.L;
@@ -653,12 +653,9 @@ int sfgpu_system::setup(const sfgpu_system_desc *d) {
         }
         store = std::max(store, need);
     }
-    if ((rc = alloc_d(&d_gi, store))) return rc;
     gi_doubles = store;
+    if (chains && (rc = alloc_chains())) return rc;
     if ((rc = alloc_d(&d_ginv[0], (size_t)K * M)) || (rc = alloc_d(&d_ginv[1], (size_t)K * M))) return rc;
-    // row-wise steps never write boundary entries; surface layers are read
-    // in place and must hold the propagator's value there, 0
-    SFGPU_CUDA_TRY(cudaMemset(d_gi, 0, sizeof(double) * std::max<size_t>(store, 1)));
     SFGPU_CUDA_TRY(cudaMemset(d_ginv[0], 0, sizeof(double) * K * M));
     SFGPU_CUDA_TRY(cudaMemset(d_ginv[1], 0, sizeof(double) * K * M));
     nblocks_red = grid_for(M);
@@ -675,6 +672,16 @@ int sfgpu_system::setup(const sfgpu_system_desc *d) {
     for (int i = 0; i < nseg; i++)
         for (int m = 0; m < nmol; m++) bp.frac[i * SFGPU_MAX_SEG + m] = (double)mols[m].count[i] / mols[m].N;
     if (d->overflow_protection) return setup_logspace();
+    return SFGPU_OK;
+}
+
+// the chain storage of residual evaluations.  Row-wise steps never write boundary
+// entries; surface layers are read in place and must hold the propagator's value
+// there, 0.
+int sfgpu_system::alloc_chains() {
+    const int rc = alloc_d(&d_gi, gi_doubles);
+    if (rc) return rc;
+    SFGPU_CUDA_TRY(cudaMemset(d_gi, 0, sizeof(double) * std::max<size_t>(gi_doubles, 1)));
     return SFGPU_OK;
 }
 
@@ -711,70 +718,55 @@ void fill_inst_desc(const sfgpu_system *s, sfb::InstDesc *out) {
     I.smap = s->d_smap; I.jall = s->d_jall; I.wpart = s->d_wpart;
 }
 
-// every molecule's segments and their runs on the device
-int sfgpu_system::upload_chains(sfb::InstDesc *I) {
-    std::vector<int> all;
-    std::vector<size_t> at(nmol);
-    for (int q = 0; q < nmol; q++) {
-        const std::vector<int> &s = mols[q].seg;
+// (1D and 2D lattices)
+void sfgpu_system::site_maps(std::vector<int> *out) const {
+    const size_t at = out->size();
+    out->resize(at + 2 * (size_t)M);
+    int *smap = out->data() + at, *jall = smap + M;
+    const int rows = H.L.grad == 2 ? H.L.Md[0] : 1, cols = M / rows;
+    for (int x = 0; x < rows; x++)
+        for (int y = 0, z = x * cols; y < cols; y++, z++) {
+            const bool edge = y == 0 || y == cols - 1 || (rows > 1 && (x == 0 || x == rows - 1));
+            smap[z] = edge ? lat_map(H.L, z) : z;
+            jall[z] = jmap_h[smap[z]];
+        }
+}
+// per molecule: segments, the end of the run of equal segments each lies in, its beginning
+void sfgpu_system::chain_tables(std::vector<int> *out) const {
+    for (const HMol &o : mols) {
+        const std::vector<int> &s = o.seg;
         const int n = (int)s.size();
-        std::vector<int> f(n), b(n);
+        const size_t at = out->size();
+        out->insert(out->end(), s.begin(), s.end());
+        out->resize(at + 3 * (size_t)n);
+        int *f = out->data() + at + n, *b = f + n;
         for (int t = n - 1; t >= 0; t--) f[t] = (t + 1 < n && s[t + 1] == s[t]) ? f[t + 1] : t + 1;
         for (int t = 0; t < n; t++) b[t] = (t > 0 && s[t - 1] == s[t]) ? b[t - 1] : t - 1;
-        at[q] = all.size();
-        all.insert(all.end(), s.begin(), s.end());
-        all.insert(all.end(), f.begin(), f.end());
-        all.insert(all.end(), b.begin(), b.end());
     }
-    int *d = nullptr;
-    const int rc = alloc_i(&d, all.size());
-    if (rc) return rc;
-    SFGPU_CUDA_TRY(cudaMemcpy(d, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice));
+}
+void sfgpu_system::point_chains(const int *d, sfb::InstDesc *I) const {
     for (int q = 0; q < nmol; q++) {
         const size_t n = mols[q].seg.size();
-        I->mol[q].seg = d + at[q];
-        I->mol[q].runf = d + at[q] + n;
-        I->mol[q].runb = d + at[q] + 2 * n;
+        I->mol[q].seg = d;
+        I->mol[q].runf = d + n;
+        I->mol[q].runb = d + 2 * n;
+        d += 3 * n;
     }
+}
+
+// Surface layers hold 0 in every state profile: the engine's contact averages of
+// a 2D lattice read them where the boundary copies are written in the same phase.
+int sfgpu_system::clear_profiles() {
+    if (H.L.grad != 2) return SFGPU_OK;
+    for (int i = 0; i < nseg; i++)
+        if (freedom[i] != SFGPU_SEG_FROZEN) SFGPU_CUDA_TRY(cudaMemset(d_phi[i], 0, sizeof(double) * M));
     return SFGPU_OK;
 }
 
-// Where the cluster engine takes the system: its index maps, its descriptor
-// on the device and its launch shape for one system alone.
+// Where the cluster engine takes the system: its launch shape for one system
+// alone, its tables and buffers, and its descriptor on the device.
 int sfgpu_system::setup_group() {
     if (!group_eligible(this)) return SFGPU_OK;
-    int rc;
-    std::vector<int> smap(M), jall(M);
-    for (int z = 0; z < M; z++) { smap[z] = lat_map(H.L, z); jall[z] = jmap_h[smap[z]]; }
-    if ((rc = alloc_i(&d_smap, M)) || (rc = alloc_i(&d_jall, M)) ||
-        (rc = alloc_d(&d_wpart, (size_t)nmol * ((M + 255) / 256))))
-        return rc;
-    SFGPU_CUDA_TRY(cudaMemcpy(d_smap, smap.data(), sizeof(int) * M, cudaMemcpyHostToDevice));
-    SFGPU_CUDA_TRY(cudaMemcpy(d_jall, jall.data(), sizeof(int) * M, cudaMemcpyHostToDevice));
-    if (H.L.grad == 1) {
-        // stored slices of whole warps, for chains that shared memory does not
-        // take; apart from d_gi, whose slices' boundary entries stay 0 for the
-        // derivatives' sweeps
-        size_t n = 0;
-        for (const auto &o : mols)
-            if (o.type != 0) n = std::max(n, (size_t)(o.sym ? o.N / 2 : o.N) * sfg::slice1d(H.L.Md[0] - 2));
-        if ((rc = alloc_d(&d_slices1, n))) return rc;
-    }
-    // surface layers hold 0 in every profile: the contact averages read them
-    // where the boundary copies are written in the same phase
-    for (int i = 0; i < nseg; i++) {
-        if (freedom[i] == SFGPU_SEG_FROZEN) continue;
-        SFGPU_CUDA_TRY(cudaMemset(d_phi[i], 0, sizeof(double) * M));
-        for (const auto &o : mols)
-            if (o.d_phi[i]) SFGPU_CUDA_TRY(cudaMemset(o.d_phi[i], 0, sizeof(double) * M));
-    }
-    std::vector<int>().swap(jmap_h);
-    group = true;
-    return SFGPU_OK;
-}
-
-// the launch shape of one system alone, and its descriptor on the device
-int sfgpu_system::setup_group_single() {
     GroupShape sh;
     bool ok = false;
     // one system alone leaves the chip idle: as many blocks as a cluster has,
@@ -786,14 +778,23 @@ int sfgpu_system::setup_group_single() {
         if (blocks == 2) break;
     }
     if (!ok) return SFGPU_OK;
+    int rc;
+    std::vector<int> tables;
+    site_maps(&tables);
+    chain_tables(&tables);
+    const size_t slices = group_slices(this, sh);
+    if ((rc = alloc_i(&d_smap, tables.size())) || (rc = alloc_d(&d_wpart, (size_t)nmol * ((M + 255) / 256))) ||
+        (slices && (rc = alloc_d(&d_slices1, slices))))
+        return rc;
+    SFGPU_CUDA_TRY(cudaMemcpy(d_smap, tables.data(), sizeof(int) * tables.size(), cudaMemcpyHostToDevice));
+    d_jall = d_smap + M;
+    if ((rc = clear_profiles())) return rc;
     sfb::InstDesc I;
     fill_inst_desc(this, &I);
-    int rc;
+    point_chains(d_smap + 2 * (size_t)M, &I);
     double *p = nullptr, *p2 = nullptr;
     const size_t nd = (sizeof(sfb::InstDesc) + 7) / 8;
-    if ((rc = upload_chains(&I)) || (rc = alloc_d(&p, nd)) || (rc = alloc_d(&p2, nd)) ||
-        (rc = alloc_i(&d_diis_int, 4)))
-        return rc;
+    if ((rc = alloc_d(&p, nd)) || (rc = alloc_d(&p2, nd)) || (rc = alloc_i(&d_diis_int, 4))) return rc;
     I.scal_out = (MolScal *)d_scal;
     I.phib_out = d_phib;
     I.chib_out = d_chib;
@@ -1701,7 +1702,7 @@ static int create_system(const sfgpu_system_desc *desc, int stride, sfgpu_system
     s->primal_stride = desc->overflow_protection ? 0 : stride;
     int rc = s->setup(desc);
     if (!rc) rc = s->setup_group();
-    if (!rc && s->group) rc = s->setup_group_single();
+    std::vector<int>().swap(s->jmap_h);
     if (!rc) rc = sfgpu_after_setup(s->stream);
     if (rc) { delete s; return rc; }
     *out = s;

@@ -199,7 +199,6 @@ struct sfgpu_system {
     // the cluster engine (sfgpu_group.cuh), where it takes this system: its
     // launch shape, the descriptor on the device and Pure_DIIS's vectors
     // (x, g and m steps twice; allocated by the first solve, then kept)
-    bool group = false;
     std::vector<int> jmap_h;
     int *d_smap = nullptr, *d_jall = nullptr;
     double *d_wpart = nullptr, *d_slices1 = nullptr;
@@ -208,16 +207,22 @@ struct sfgpu_system {
     double *d_diis = nullptr;
     int diis_m = 0;
     int *d_diis_int = nullptr;
-    int upload_chains(sfb::InstDesc *I);
+    // host tables of the engine and of the batch kernel: per site the site it
+    // copies, then that site's iteration index; every molecule's segments and runs
+    void site_maps(std::vector<int> *out) const;
+    void chain_tables(std::vector<int> *out) const;
+    void point_chains(const int *d, sfb::InstDesc *I) const;
+    int clear_profiles();
     int setup_group();
-    int setup_group_single();
     int solve_group(double *x, double tol, int maxit, int m, double eta, int *iterations, double *final_error);
     std::vector<void *> allocs;
 
     ~sfgpu_system();
     int alloc_d(double **p, size_t n);
     int alloc_i(int **p, size_t n);
-    int setup(const sfgpu_system_desc *d);
+    // chains: with the chain storage d_gi, else alloc_chains() takes it later
+    int setup(const sfgpu_system_desc *d, bool chains = true);
+    int alloc_chains();
     int molecule_phi(int m);
     int residual_async(const double *x, double *f);
     int free_energy(double *F);
