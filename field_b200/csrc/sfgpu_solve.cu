@@ -191,6 +191,7 @@ extern "C" int sfgpu_solve_diis_many(int n, sfgpu_system *const *systems, double
             int it = 0;
             double err = 0;
             status[i] = sfgpu_solve_diis(systems[i], x[i], tol, maxit, m, eta, &it, &err);
+            systems[i]->release_diis();   // of as many systems at a time as there are threads
             if (iterations) iterations[i] = it;
             if (errors) errors[i] = err;
         }

@@ -198,7 +198,7 @@ struct sfgpu_system {
     int setup_charges(const sfgpu_system_desc *d, const std::vector<int> &jmap);
     // the cluster engine (sfgpu_group.cuh), where it takes this system: its
     // launch shape, the descriptor on the device and Pure_DIIS's vectors
-    // (x, g and m steps twice; allocated by the first solve, then kept)
+    // (x, g and m steps twice; allocated by a solve and kept up to kDiisKept bytes)
     std::vector<int> jmap_h;
     int *d_smap = nullptr, *d_jall = nullptr;
     double *d_wpart = nullptr, *d_slices1 = nullptr;
@@ -214,6 +214,7 @@ struct sfgpu_system {
     void point_chains(const int *d, sfb::InstDesc *I) const;
     int clear_profiles();
     int setup_group();
+    void release_diis();
     int solve_group(double *x, double tol, int maxit, int m, double eta, int *iterations, double *final_error);
     std::vector<void *> allocs;
 
