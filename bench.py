@@ -266,9 +266,8 @@ def run_reference(a, rank, world):
 
 # ---------------------------------------------------------------------------
 def plain_form(config, insts, stream, steps=1):
-    """Per-instance host-driven GPU form: Pure_DIIS with one launch per
-    propagator step on the cylinder, SFbox's Newton iteration over the device
-    residual on the 1D instances.  Returns (solves/s, a System, iterations,
+    """Per-instance GPU form: Pure_DIIS on the cylinder, SFbox's Newton iteration
+    over the device residual on the 1D instances.  Returns (solves/s, a System, iterations,
     converged)."""
     import torch
     from field_b200.system import System
@@ -399,12 +398,14 @@ def run_ours(a, rank, world, local_rank):
     if a.form == "chosen":
         ns = min(a.plain_sample, len(insts))
         pv, prof_sys, _, pconv = plain_form(cfg, insts[:ns], stream, steps=1)
+        solve = "one launch per solve" if prof_sys.one_launch else "one launch per propagator step"
         plain = {"value": pv, "unit": "solves/s", "instances": ns, "converged": int(pconv),
-                 "form": ("per-instance Pure_DIIS, one launch per solve" if cfg == "c2" else
+                 "form": (f"per-instance Pure_DIIS, {solve}" if cfg == "c2" else
                           "per-instance SFbox Newton iteration (pseudohessian, Scheutjens step search) "
                           "over the device residual, host-driven")}
         kp_bytes = solver.algorithmic_bytes(last_iters)
-        prof_k = {"kernel": "group_diis_kernel (a cluster per instance, one launch per batch solve)",
+        kernel = "group_diis_kernel (a cluster" if solver.cluster else "batch_diis_kernel (a block"
+        prof_k = {"kernel": kernel + " per instance, one launch per batch solve)",
                   "bytes": kp_bytes, "ms": statistics.median(kms)}
         solver.kernel_profile = prof_k
     prof = prof_sys.profile_propagator(reps=400)
@@ -426,7 +427,8 @@ def run_ours(a, rank, world, local_rank):
                 "e2e": e2e, "roofline": roof, "plain_gpu_form": plain,
                 "chosen_over_plain": (value / plain["value"]) if plain and plain["value"] > 0 else None,
                 "cpu_baseline": cpu, "clocks": clocks,
-                "gpu_launches": fbatch.launch_count(a.form, iters_total, [(s, x) for s, x, _ in insts], solver)}
+                "gpu_launches": fbatch.launch_count(a.form, iters_total, [(s, x) for s, x, _ in insts], solver,
+                                                     prof_sys)}
         print(json.dumps(line), flush=True)
 
 

@@ -67,7 +67,9 @@ PROTOTYPES = {
     "sfgpu_batch_destroy": (i32, [vp]),
     "sfgpu_batch_info": (i32, [vp, ip, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]),
     "sfgpu_batch_set_stream": (i32, [vp, vp]),
+    "sfgpu_system_one_launch": (i32, [vp, ip]),
     "sfgpu_batch_set_launch": (i32, [vp, i32, i32]),
+    "sfgpu_batch_cluster": (i32, [vp, ip, ip]),
     "sfgpu_batch_solve": (i32, [vp, dp, dp, f64, i32, f64, ip, ip, dp]),
     "sfgpu_batch_get_phi": (i32, [vp, i32, i32, dp]),
     "sfgpu_batch_load": (i32, [vp, dp]),

@@ -29,24 +29,12 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-def one_launch(spec) -> bool:
-    """Whether the cluster engine evaluates (and iterates) the system in one
-    launch: linear first-order chains on 1D and 2D lattices (group_eligible in
-    csrc/sfgpu_group.cu)."""
-    lat = spec.lattice
-    n = lat.n_layers[:lat.gradients]
-    if lat.order != 1 or lat.gradients > 2 or spec.overflow_protection or spec.charged or min(n) < 3:
-        return False
-    if any(m.generations or m.bond_parent is not None or m.ring or m.force for m in spec.molecules):
-        return False
-    return lat.gradients == 2 or (4 not in (lat.bound_lo[0], lat.bound_hi[0]) and n[0] <= 1664)
-
-
-def launches_per_residual(spec) -> int:
+def launches_per_residual(spec, system=None) -> int:
     """Kernel launches of one single-system residual evaluation
-    (sfgpu_system::residual_async): SWF updates, per-molecule propagation,
-    state sums, bulk scalars and the residual kernel."""
-    if one_launch(spec):
+    (sfgpu_system::residual_async): 1 where ``system`` (the spec's System) runs
+    in the cluster engine, else SWF updates, per-molecule propagation, state
+    sums, bulk scalars and the residual kernel."""
+    if system is not None and system.one_launch:
         return 1
     K = spec.lattice.components
     n = 0
@@ -66,11 +54,11 @@ def launches_per_residual(spec) -> int:
     return n + 2
 
 
-def launch_count(form: str, iterations_total: int, insts, solver=None) -> int:
+def launch_count(form: str, iterations_total: int, insts, solver=None, system=None) -> int:
     if form == "chosen" and solver is not None:
         return solver.launches_in_last_solve_total
     n_inst = len(insts)
-    if one_launch(insts[0][0]):
+    if system is not None and system.one_launch:
         return n_inst   # a solve is one launch
     per = launches_per_residual(insts[0][0])
     # per DIIS iteration: residual + step + dots + sum + combine; plus the start
@@ -147,6 +135,9 @@ class BatchSolver:
         offs = (C.c_longlong * len(self.specs))()
         nat.check(self.lib.sfgpu_batch_info(h, C.byref(n), C.byref(tot), offs), "sfgpu_batch_info")
         self.n, self.total = n.value, tot.value
+        blocks = C.c_int()
+        nat.check(self.lib.sfgpu_batch_cluster(h, C.byref(blocks), None), "sfgpu_batch_cluster")
+        self.cluster = blocks.value     # blocks per instance in the cluster engine, 0 outside it
         self.offsets = np.array(list(offs), dtype=np.int64)
         self.launches_in_last_solve_total = 0
         self.kernel_profile = None
@@ -189,13 +180,19 @@ class BatchSolver:
 
     def set_launch(self, threads: int, stage: bool = True):
         """Threads per block and shared-memory staging of the persistent
-        kernel (sfgpu_batch_set_launch)."""
+        kernel (sfgpu_batch_set_launch); batches of the cluster engine
+        (``cluster`` > 0) keep the engine's shape."""
         nat.check(self.lib.sfgpu_batch_set_launch(self.h, int(threads), int(bool(stage))), "sfgpu_batch_set_launch")
 
     def autotune(self, x0, tol=1e-7, maxit=2000, candidates=((1024, True), (512, True), (512, False),
                                                              (384, True), (256, True))):
         """Time one solve per launch shape from x0 and keep the fastest;
-        returns {(threads, stage): ms}."""
+        returns {(threads, stage): ms}.  A batch of the cluster engine has one
+        shape, the engine's."""
+        if self.cluster:
+            th = C.c_int()
+            nat.check(self.lib.sfgpu_batch_cluster(self.h, None, C.byref(th)), "sfgpu_batch_cluster")
+            candidates = ((th.value, True),)
         times = {}
         for th, stg in candidates:
             try:

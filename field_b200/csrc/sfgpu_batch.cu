@@ -298,6 +298,13 @@ extern "C" int sfgpu_batch_set_stream(sfgpu_batch *b, void *stream) {
     return SFGPU_OK;
 }
 
+extern "C" int sfgpu_batch_cluster(sfgpu_batch *b, int *blocks, int *threads) {
+    if (!b) return SFGPU_ERR_INVALID;
+    if (blocks) *blocks = b->grouped ? b->shape.C : 0;
+    if (threads) *threads = b->grouped ? b->shape.threads : b->block;
+    return SFGPU_OK;
+}
+
 // Launch shape of the persistent kernel: threads per block (32..1024, a
 // multiple of 32) and whether instances stage G (and the 1D slices) in
 // shared memory.  By default 1024/512/256 threads by lattice size and

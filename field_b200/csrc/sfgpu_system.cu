@@ -2113,6 +2113,13 @@ extern "C" int sfgpu_system_autotune(sfgpu_system *s, int reps, int *chosen_xc, 
     return SFGPU_OK;
 }
 
+extern "C" int sfgpu_system_one_launch(sfgpu_system *s, int *one) {
+    CHECK_SYS(s);
+    if (!one) return fail(SFGPU_ERR_INVALID, "null argument");
+    *one = s->group_shape_ != nullptr;
+    return SFGPU_OK;
+}
+
 extern "C" int sfgpu_system_set_tile_pipelined(sfgpu_system *s, int enable) {
     CHECK_SYS(s);
     if (enable < 0 || enable > 2) return fail(SFGPU_ERR_INVALID, "the step form is 0, 1 or 2");

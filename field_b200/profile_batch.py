@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import sys
 
 import numpy as np
 
@@ -33,14 +34,16 @@ def main():
         insts = configs.sweep1d(count=256)[:a.instances]
         m, maxit = 5, 5000
     bs = BatchSolver([s for s, _ in insts], m=m, eta=0.1)
-    if a.threads:
+    if a.threads and bs.cluster:
+        print("the cluster engine sets its own launch shape: --threads has no effect here", file=sys.stderr)
+    elif a.threads:
         bs.set_launch(a.threads, True)
     x = np.concatenate([x for _, x in insts])
     for _ in range(2):
         bs.load(x)
         bs.solve_resident(1e-7, maxit)
         r = bs.results()
-    print(json.dumps({"case": a.case, "instances": a.instances, "kernel_ms": bs.kernel_ms(),
+    print(json.dumps({"case": a.case, "instances": a.instances, "cluster": bs.cluster, "kernel_ms": bs.kernel_ms(),
                       "converged": int(r.converged.sum()), "mean_iterations": float(np.mean(r.iterations))}))
 
 

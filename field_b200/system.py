@@ -263,6 +263,14 @@ class System:
                   "sfgpu_profile_propagator")
         return {"ms_fwd": a.value, "ms_bwd": b.value, "bytes_fwd": c.value, "bytes_bwd": d.value}
 
+    @property
+    def one_launch(self) -> bool:
+        """Whether the cluster engine evaluates the system: one launch per
+        residual, and per solve with m <= 16 (sfgpu_system_one_launch)."""
+        v = C.c_int()
+        nat.check(self.lib.sfgpu_system_one_launch(self.h, C.byref(v)), "sfgpu_system_one_launch")
+        return bool(v.value)
+
     def autotune(self, reps: int = 20):
         x, ms = C.c_int(), C.c_double()
         nat.check(self.lib.sfgpu_system_autotune(self.h, reps, C.byref(x), C.byref(ms)), "sfgpu_system_autotune")

@@ -448,6 +448,10 @@ int sfgpu_system_set_tile(sfgpu_system *sys, int xc);
  * sfgpu_system_set_tile (which selects a march) and this call set both kinds. */
 int sfgpu_system_set_tile_pipelined(sfgpu_system *sys, int enable);
 int sfgpu_system_autotune(sfgpu_system *sys, int reps, int *chosen_xc, double *best_ms);
+/* *one = 1 when the cluster engine evaluates the system: a residual is one
+ * launch, and so is a Pure_DIIS solve with m <= 16; 0 when it is a launch per
+ * propagator step. */
+int sfgpu_system_one_launch(sfgpu_system *sys, int *one);
 
 /* ---- iterations ------------------------------------------------------- */
 /* Many systems solved at once, each by sfgpu_solve_diis on its own stream
@@ -521,10 +525,14 @@ int sfgpu_batch_set_stream(sfgpu_batch *batch, void *stream);
  * the running segment (and on 1D symmetric homopolymers the running slices,
  * phi and a ring of stored slices) is staged in shared memory (default 1).
  * Batches of linear chains on 1D or 2D lattices of one geometry run a
- * thread-block cluster per instance, whose shape this call leaves as it is.
- * Results do not depend on it; the autotuner of field_b200.batch times the
- * candidates. */
+ * thread-block cluster per instance, whose shape this call leaves as it is
+ * (sfgpu_batch_cluster tells).  Results do not depend on it; the autotuner of
+ * field_b200.batch times the candidates. */
 int sfgpu_batch_set_launch(sfgpu_batch *batch, int threads, int stage);
+/* the cluster engine's shape for the batch: blocks of an instance's cluster and
+ * threads of a block; 0 blocks when the batch runs a block per instance, of the
+ * threads sfgpu_batch_set_launch sets.  Either pointer may be NULL. */
+int sfgpu_batch_cluster(sfgpu_batch *batch, int *blocks, int *threads);
 /* Pure_DIIS (SFNewton::PlainLBFGSDIIS, sfnewton.cpp:566-664) on every
  * instance in one persistent kernel launch: thread blocks take instances
  * from a work queue and iterate them to |f| <= tol on the device.  x_in is
