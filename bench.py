@@ -428,7 +428,7 @@ def run_ours(a, rank, world, local_rank):
                 "chosen_over_plain": (value / plain["value"]) if plain and plain["value"] > 0 else None,
                 "cpu_baseline": cpu, "clocks": clocks,
                 "gpu_launches": fbatch.launch_count(a.form, iters_total, [(s, x) for s, x, _ in insts], solver,
-                                                     prof_sys)}
+                                                     prof_sys, newton=cfg == "c4")}
         print(json.dumps(line), flush=True)
 
 

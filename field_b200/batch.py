@@ -54,12 +54,13 @@ def launches_per_residual(spec, system=None) -> int:
     return n + 2
 
 
-def launch_count(form: str, iterations_total: int, insts, solver=None, system=None) -> int:
+def launch_count(form: str, iterations_total: int, insts, solver=None, system=None, newton=False) -> int:
     if form == "chosen" and solver is not None:
         return solver.launches_in_last_solve_total
     n_inst = len(insts)
     if system is not None and system.one_launch:
-        return n_inst   # a solve is one launch
+        # a Pure_DIIS solve is one launch, a Newton iteration one residual at least
+        return iterations_total + n_inst if newton else n_inst
     per = launches_per_residual(insts[0][0])
     # per DIIS iteration: residual + step + dots + sum + combine; plus the start
     return iterations_total * (per + 4) + n_inst * (per + 3)
@@ -70,8 +71,8 @@ def roofline(prof: dict, form: str, solver=None) -> dict:
     if form == "chosen" and solver is not None and getattr(solver, "kernel_profile", None):
         kp = solver.kernel_profile
         ach = kp["bytes"] / (kp["ms"] / 1e3) / 1e9
-        return {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                "traffic": None,
+        return {"bound": "latency" if solver.cluster else "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+                "frac": ach / peak, "traffic": None,
                 "peak_kind": kind, "kernel": kp["kernel"],
                 "bytes_per_launch": kp["bytes"], "ms_per_launch": kp["ms"]}
     ach = prof["bytes_bwd"] / (prof["ms_bwd"] / 1e3) / 1e9
@@ -112,6 +113,26 @@ def residual_bytes(spec) -> float:
             nf, nb = N - 1, N - 1
         tot += nf * 8.0 * (2 * K + 1) * M + nb * 8.0 * (3 * K + 3) * M
     return tot
+
+
+def engine_bytes(spec, iterations: int, m: int) -> float:
+    """Bytes one Pure_DIIS solve of ``iterations`` iterations moves in the
+    cluster engine (csrc/sfgpu_group.cuh), where the running slice, G and phi of
+    the running segment stay on chip.  2D: per evaluation each forward slice
+    written and read once (16 a site and segment; a symmetric homopolymer's half
+    chain), x read and f written; per iteration x, f and the kept steps read, the
+    new step and x written, XR read for the combination.  1D: the guess in and the
+    iterate out, as everything that fits lies in shared memory."""
+    nv = spec.n_itvar()
+    if spec.lattice.gradients == 1:
+        return 16.0 * nv
+    slices = 0
+    for mol in spec.molecules:
+        if mol.N > 1:
+            slices += mol.N // 2 if len({b[0] for b in mol.blocks}) == 1 else mol.N
+    kept = sum(min(i + 1, m) for i in range(1, iterations + 1))
+    return ((iterations + 1) * 16.0 * (slices * spec.M + nv) +
+            8.0 * nv * (2 * kept + 4 * iterations) + 8.0 * nv * 5)
 
 
 class BatchSolver:
@@ -241,7 +262,10 @@ class BatchSolver:
         return out
 
     def algorithmic_bytes(self, iterations) -> float:
-        """Propagator bytes plus DIIS vector traffic of one batch solve."""
+        """Bytes of one batch solve: engine_bytes in the cluster engine, else
+        propagator bytes plus DIIS vector traffic."""
+        if self.cluster:
+            return sum(engine_bytes(sp, int(it), self.m) for sp, it in zip(self.specs, iterations))
         tot = 0.0
         for sp, it in zip(self.specs, iterations):
             nv = sp.n_itvar()
