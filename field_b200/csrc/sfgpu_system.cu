@@ -2122,9 +2122,9 @@ extern "C" int sfgpu_system_one_launch(sfgpu_system *s, int *one) {
 
 extern "C" int sfgpu_system_set_tile_pipelined(sfgpu_system *s, int enable) {
     CHECK_SYS(s);
-    if (enable < 0 || enable > 2) return fail(SFGPU_ERR_INVALID, "the step form is 0, 1 or 2");
+    if (enable < 0 || enable > 3) return fail(SFGPU_ERR_INVALID, "the step form is 0, 1, 2 or 3");
     s->tile_pipelined = enable;
-    s->tile_pipelined_bwd = enable != 0;
+    s->tile_pipelined_bwd = enable == 2 ? 1 : enable;
     return SFGPU_OK;
 }
 

@@ -26,8 +26,8 @@ def main():
     ap.add_argument("--reps", type=int, default=50)
     ap.add_argument("--n", type=int, default=0, help="lattice size override")
     ap.add_argument("--tile", type=int, default=0, help="3D x-chunk depth (0: autotune)")
-    ap.add_argument("--form", default="pipelined", choices=["pipelined", "plain", "pipelined2"],
-                    help="3D first-order step form when --tile is given")
+    ap.add_argument("--form", default="pipelined", choices=["pipelined", "plain", "pipelined2", "columns"],
+                    help="3D first-order step form when --tile is given (columns have no depth)")
     a = ap.parse_args()
     if a.case == "c2":
         spec, x = configs.cyl_micelle(**({"nx": a.n, "ny": a.n} if a.n else {}))
@@ -40,7 +40,7 @@ def main():
     tune = None
     if a.tile:
         s.set_tile(a.tile)
-        s.set_tile_pipelined({"plain": 0, "pipelined": 1, "pipelined2": 2}[a.form])
+        s.set_tile_pipelined({"plain": 0, "pipelined": 1, "pipelined2": 2, "columns": 3}[a.form])
     else:
         tune = s.autotune(reps=max(5, a.reps // 5))
     p = s.profile_propagator(reps=a.reps)

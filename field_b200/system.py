@@ -277,9 +277,9 @@ class System:
         return {"tile_xc": x.value, "ms_fwd_plus_bwd": ms.value}
 
     def set_tile_pipelined(self, enable):
-        """March form of the 3D first-order step in place of the default column
-        form: False/0 plain, True/1 pipelined, 2 pipelined with two y rows per
-        thread in the forward steps."""
+        """Form of the 3D first-order step: 3 columns (the default); marches:
+        False/0 plain, True/1 pipelined, 2 pipelined with two y rows per thread
+        in the forward steps."""
         nat.check(self.lib.sfgpu_system_set_tile_pipelined(self.h, int(enable)), "set_tile_pipelined")
 
     def set_tile(self, xc: int):

@@ -439,12 +439,12 @@ int sfgpu_profile_propagator(sfgpu_system *sys, int reps, double *ms_fwd, double
  * buffers and keep the fastest (reps forward + backward steps each; the
  * propagator contents are overwritten).  Other lattices ignore it. */
 int sfgpu_system_set_tile(sfgpu_system *sys, int xc);
-/* March forms of the 3D first-order step.  1: software-pipelined (plane x+1's
- * loads in flight while plane x is computed, double-buffered tile); 0: the
- * plain x-marching form; 2: pipelined, the forward (composition-free) steps
- * with two y rows of columns per thread.  By default no march runs: a thread
- * owns four planes of one column.  Results are bit-identical.  The autotuner
- * times every form, and the marches' depths, for each kind of step.
+/* Form of the 3D first-order step.  3, the default: no march, a thread owns four
+ * planes of one column.  March forms: 1 software-pipelined (plane x+1's loads in
+ * flight while plane x is computed, double-buffered tile); 0 the plain
+ * x-marching form; 2 pipelined, the forward (composition-free) steps with two y
+ * rows of columns per thread.  Results are bit-identical.  The autotuner times
+ * every form, and the marches' depths, for each kind of step.
  * sfgpu_system_set_tile (which selects a march) and this call set both kinds. */
 int sfgpu_system_set_tile_pipelined(sfgpu_system *sys, int enable);
 int sfgpu_system_autotune(sfgpu_system *sys, int reps, int *chosen_xc, double *best_ms);

@@ -37,3 +37,19 @@ def test_columns(n, lo, hi):
     assert np.array_equal(fj, f)
     _, jw = s.vjp(x, w)
     assert abs(w @ jv - jw @ v) <= 1e-10 * np.linalg.norm(w) * np.linalg.norm(jv)
+
+
+def test_the_default_form_can_be_set_again():
+    from field_b200 import _native
+    from field_b200.configs import melt3d
+    from field_b200.system import System
+    spec, x = melt3d(n=40, nA=10, nB=10)
+    s = System(spec)
+    f = s.residual(x)
+    s.set_tile(4)
+    s.set_tile_pipelined(1)
+    assert np.array_equal(s.residual(x), f)
+    s.set_tile_pipelined(3)
+    assert np.array_equal(s.residual(x), f)
+    with pytest.raises(_native.SfgpuError):
+        s.set_tile_pipelined(4)
