@@ -95,9 +95,11 @@ static int configure_stage(sfgpu_batch *b, bool allow) {
 // The cluster engine takes a batch whose instances it all accepts on lattices
 // of one kind.  2D blocks per instance: with enough instances to fill the
 // chip, about 2048 sites a block (fewer blocks idle less in halo exchanges,
-// more let two blocks share an SM and hide them); 296 cylinders of 128 x 128
+// more let two blocks share an SM and hide them).  296 cylinders of 128 x 128
 // to 1e-11: 172 ms with 8 blocks of 256 threads, 176 with 4 of 512, 218 with 16
-// of 256, and 231 in the one-block-per-instance kernel.  With fewer instances
+// of 256, and 231 in the one-block-per-instance kernel; these with the engine as
+// it was before the phases that run once an iteration were shortened, with
+// which the 8 blocks take 159.  With fewer instances
 // the SMs left over go to their clusters.
 static void configure_group(sfgpu_batch *b) {
     const sfgpu_system *s0 = b->sys[0];

@@ -308,8 +308,9 @@ bool group_shape(const sfgpu_system *s, int blocks, int threads, int m, GroupSha
         g.C = 1;
         g.J = 1;
         // the phases between the chains want a thread per site (one system alone,
-        // n = 200: 3.30 ms a solve with 128 threads, 2.95 with 256); two blocks
-        // share an SM in a large batch, whose registers then hold 128 each
+        // n = 200: 3.30 ms a solve with 128 threads, 2.95 with 256).  In a large
+        // batch two blocks of 128 share an SM where the largest instance leaves
+        // them the room: up to 96 KB each beside 17 KB of static shared memory
         g.threads = std::max(blocks > 1 ? 256 : 128, 32 * warps1d(n));
         // what localize1d takes, in its order; the last ones only where they fit
         const Doubles1 need = doubles1(s);

@@ -12,13 +12,15 @@
 // with cluster barriers between the phases.
 //
 // What bounds it is latency, not traffic.  Measured on a B200 against the
-// launch-per-step path (microseconds):
-//   residual, 1D n = 100, N = 100            269 -> 27    (0.09 a step, of which 0.045
+// launch-per-step path (microseconds; both builds in turn on one box):
+//   residual, 1D n = 100, N = 100            222 -> 26.6  (0.09 a step, of which 0.045
 //                                                          are the shuffle and the step's
 //                                                          six dependent FP64 operations)
-//   residual, 2D cylinder 128 x 128, N = 40  334 -> 72    (0.43 a step)
-//   Pure_DIIS, 1D n = 200, N = 200         32000 -> 2900
-//   Pure_DIIS, 2D cylinder 128 x 128       28000 -> 4700
+//   residual, 2D cylinder 128 x 128, N = 40  335 -> 71    (0.43 a step)
+//   Pure_DIIS, 1D n = 200, N = 200         40053 -> 3067
+//   Pure_DIIS, 2D cylinder 128 x 128       18289 -> 4121
+// Of an issued instruction's 11 cycles in the 2D residual 2.6 are barriers, 2.1
+// fixed latencies, 1.7 loads and 1.2 instruction fetches.
 //
 // Every value is formed by the operations, in the order, of the
 // single-system kernels (stencil1, finalize_phi, residual) and lnGN sums run
@@ -513,9 +515,10 @@ __device__ __noinline__ void chain2d(const InstDesc &I, int m, const Grp &gr, GS
 // Position 0 is the first register of some lane of warp 0 and position n + 1
 // lies in the last warp; G is 0 there, so a surface layer's value stays 0 and
 // only mirrors need a rule.  Lattices wider than one warp are cut into runs of
-// kOwn1 positions with kHalo1 further ones on either side that a warp
-// recomputes; after kHalo1 steps the warps exchange their values once through
-// shared memory.
+// kOwn1 positions, with kHalo1 + 1 further ones below and kHalo1 - 1 above that a
+// warp recomputes (position 0 has to be some lane's first register).  A step
+// makes one more position at either end wrong, so after kHalo1 - 1 steps the
+// warps exchange their values once through shared memory.
 //
 // One warp walks the chain alone, so a step is a latency: the loops are short
 // and free of branches (an eight-fold unrolled form with a rule per boundary

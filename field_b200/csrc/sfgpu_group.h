@@ -4,9 +4,12 @@
 #include "sfgpu_system.h"
 
 namespace sfg {
-// 1D chains: a warp's sites per lane, the sites it recomputes on either side
-// of its own, and its own; stored slices are whole warps of lanes
+// 1D chains: a warp's sites per lane, and its own ones; it recomputes kHalo1 + 1
+// sites below them and kHalo1 - 1 above, which are right for as many steps.
+// Stored slices are whole warps of lanes.
 constexpr int kJ1 = 4, kHalo1 = 12, kOwn1 = 32 * kJ1 - 2 * kHalo1;
+static_assert(kHalo1 % kJ1 == 0, "position 0 is the first register of a lane");
+static_assert(32 * kJ1 - (kHalo1 + 1) - kOwn1 >= kHalo1 - 1, "sites above a warp's own, one for each step between exchanges");
 constexpr int kMaxWarps1 = 16;
 constexpr int kRing1 = 8;       // stored slices on their way back from global memory (a power of two)
 __host__ __device__ inline int warps1d(int n) { return n <= 32 * kJ1 - 2 ? 1 : (n + kOwn1 - 1) / kOwn1; }

@@ -730,9 +730,11 @@ step2_rows(DLat L, const double *__restrict__ gin, const double *__restrict__ G,
 // 32 (z) x 2 (y) x 2 (x) sites.  Same weights and summation order as comp2.
 // Measured against a warp per row (us): 96^3 forward 23.7 -> 23.2, composing
 // 28.1 -> 25.3 (6.2 TB/s of algorithmic bytes); 50 x 40 x 45 5.9 -> 5.4, 5.0 -> 4.4.
-// Block shapes from 32 x 4 x 1 to 32 x 2 x 8 lie within 4 % of one another: the
-// forward step is not held by the reads that neighbours share but by the 45 MB
-// slice it writes to memory beside the one it reads from L2.
+// The forward step is the slower one for its bytes: it pulls five components from
+// each of six neighbours, 30 loads a site, so a block reads nearly all components
+// of its whole halo and the slice crosses L2 about three times; the backward step
+// reads each component from one site.  Block shapes from 32 x 4 x 1 to 32 x 2 x 8
+// lie within 4 % of one another, as all of them pull.
 // The offsets and mirror flags are formed before pdl_enter(), while the previous
 // step drains (whole residual, 40 segments, us): 16^3 341 -> 305 (a warp per row
 // 322), 60 x 60 x 40 634 -> 561, 96 x 96 x 16 680 -> 579.
